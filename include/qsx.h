@@ -357,7 +357,9 @@ typedef struct {
   double* out_proj;       /* complex128 [batch][nsave][nout] or NULL */
   double* out_mean;       /* complex128 [nsave][nout] or NULL */
   double mean_scale;      /* out_mean = mean_scale * sum over samples */
-  void* workspace;        /* scratch for out_mean partial sums */
+  void* workspace;        /* scratch for out_mean partial sums; for out_state
+                             alone, optional scratch that lets few samples run
+                             by doubling (16-byte aligned) */
   size_t workspace_bytes;
   int32_t* status;        /* device int: set to QSX_ERR_NONFINITE on NaN/Inf */
   int32_t variant;        /* kernel variant, 0 = the planner's choice; with block_k:

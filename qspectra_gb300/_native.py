@@ -837,7 +837,7 @@ def rk4(matrix, y0, nsteps, save_every=1, form=0, h=0.0, precision=None,
     status = torch.zeros(1, dtype=torch.int32, device=dev)
     a.status = status.data_ptr()
     lib = load()
-    if mean and nout:
+    if (mean and nout) or state:
         nbytes = ctypes.c_size_t(0)
         _check(lib.qsx_rk4_workspace_bytes(ctypes.byref(a), ctypes.byref(nbytes)),
                'qsx_rk4_workspace_bytes')

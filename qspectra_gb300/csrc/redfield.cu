@@ -8,6 +8,7 @@
 #include <type_traits>
 
 #include "qsx_common.cuh"
+#include "rk4_traj.cuh"
 
 namespace qsx {
 
@@ -1624,8 +1625,16 @@ int qsx_rk4_propagator_batched(const double* L, int m, int64_t batch, double h,
     propagator_kernel<float><<<(unsigned)batch, 256, smem, s>>>((const double2*)L, m, h,
                                                                 (float2*)D);
   } else {
+    // a CTA per row while the extra product of that form (half as much work
+    // again) is less than the SMs that one CTA per sample leaves idle
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return cuda_status(e, "qsx_rk4_propagator_batched");
+    if (3 * batch <= 2 * (int64_t)sms)
+      return propagator_rows_run((const double2*)L, m, batch, h, (double2*)D, s);
     size_t smem = 3 * mm * sizeof(double2);
-    cudaError_t e = cudaFuncSetAttribute(propagator_kernel<double>,
+    e = cudaFuncSetAttribute(propagator_kernel<double>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_status(e, "qsx_rk4_propagator_batched");
     propagator_kernel<double><<<(unsigned)batch, 256, smem, s>>>((const double2*)L, m, h,

@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "qsx_common.cuh"
+#include "rk4_traj.cuh"
 
 namespace qsx {
 
@@ -37,6 +38,7 @@ struct Rk4P {
   double2* partial;   // generic kernel: [nslots][nsave][nout] double2, or null
   float2* partial32;  // FP32 kernels: [nslots][nsave][nout] float2, or null
   int* status;
+  const int* only_if;  // generic kernel: run only when this device word is nonzero (null: always)
 };
 
 __device__ __forceinline__ float2 f2(double2 v) { return make_float2((float)v.x, (float)v.y); }
@@ -708,6 +710,7 @@ __global__ void __launch_bounds__(1024) rk4_generic(Rk4P p, int mat_in_smem) {
   using C = typename cplx<T>::type;
   constexpr bool SPLIT = sizeof(T) == 4;
   extern __shared__ __align__(16) unsigned char sm[];
+  if (p.only_if && *p.only_if == 0) return;
   const int M = p.m;
   double2* red = (double2*)sm;      // [32] block reduction (16-byte aligned first)
   C* ybuf = (C*)(red + 32);         // [2][M] current state (hi) / stage input
@@ -950,6 +953,22 @@ static int validate(const qsx_rk4_args* a) {
   return QSX_OK;
 }
 
+static int generic_plan(const qsx_rk4_args* a, Plan* pl) {
+  const int m = a->m;
+  pl->kind = K_GENERIC;
+  int nt = ((std::min(m, 1024) + 31) / 32) * 32;
+  QSX_CHECK_ARG((m + nt - 1) / nt <= GEN_MAXR, "qsx_rk4: m too large");
+  pl->threads = nt;
+  pl->grid = a->batch;
+  pl->nslots = a->batch;
+  size_t cs = a->precision == QSX_FP32 ? sizeof(float2) : sizeof(double2);
+  size_t base = 2 * (size_t)m * cs + 32 * sizeof(double2);
+  size_t mat = (size_t)m * m * cs;
+  pl->mat_in_smem = (base + mat) <= 160 * 1024;
+  pl->smem = base + (pl->mat_in_smem ? mat : 0);
+  return QSX_OK;
+}
+
 static int make_plan(const qsx_rk4_args* a, Plan* pl) {
   int G = 0;
   const int m = a->m;
@@ -1051,18 +1070,7 @@ static int make_plan(const qsx_rk4_args* a, Plan* pl) {
       return QSX_OK;
     }
   }
-  pl->kind = K_GENERIC;
-  int nt = ((std::min(m, 1024) + 31) / 32) * 32;
-  QSX_CHECK_ARG((m + nt - 1) / nt <= GEN_MAXR, "qsx_rk4: m too large");
-  pl->threads = nt;
-  pl->grid = a->batch;
-  pl->nslots = a->batch;
-  size_t cs = a->precision == QSX_FP32 ? sizeof(float2) : sizeof(double2);
-  size_t base = 2 * (size_t)m * cs + 32 * sizeof(double2);
-  size_t mat = (size_t)m * m * cs;
-  pl->mat_in_smem = (base + mat) <= 160 * 1024;
-  pl->smem = base + (pl->mat_in_smem ? mat : 0);
-  return QSX_OK;
+  return generic_plan(a, pl);
 }
 
 }  // namespace qsx
@@ -1078,7 +1086,13 @@ int qsx_rk4_workspace_bytes(const qsx_rk4_args* a, size_t* bytes) {
   if (st) return st;
   QSX_CHECK_ARG(bytes != nullptr, "qsx_rk4_workspace_bytes: null output");
   *bytes = 0;
-  if (a->out_mean == nullptr || a->batch == 0) return QSX_OK;
+  if (a->batch == 0) return QSX_OK;
+  if (a->out_mean == nullptr) {
+    TrajPlan tr;
+    st = rk4_traj_plan(a, &tr);
+    if (st == QSX_OK && tr.form != TRAJ_NONE) *bytes = tr.bytes;
+    return st;
+  }
   Plan pl;
   st = make_plan(a, &pl);
   if (st) return st;
@@ -1092,11 +1106,25 @@ int qsx_rk4_batched(const qsx_rk4_args* a, void* stream) {
   int st = validate(a);
   if (st) return st;
   if (a->batch == 0) return QSX_OK;
-  Plan pl;
-  st = make_plan(a, &pl);
-  if (st) return st;
   cudaStream_t s = (cudaStream_t)stream;
+  Plan pl;
   Rk4P p;
+  p.only_if = nullptr;
+  // few samples with every state wanted: by doubling, given the workspace
+  TrajPlan tr;
+  st = rk4_traj_plan(a, &tr);
+  if (st) return st;
+  if (tr.form != TRAJ_NONE && a->workspace && a->workspace_bytes >= tr.bytes &&
+      ((uintptr_t)a->workspace & 15) == 0) {
+    st = rk4_traj_run(a, tr, s);
+    if (st) return st;
+    // the stepped loop, if a power or a state was not finite
+    p.only_if = (const int*)a->workspace;
+    st = generic_plan(a, &pl);
+  } else {
+    st = make_plan(a, &pl);
+  }
+  if (st) return st;
   p.m = a->m;
   p.nsteps = a->nsteps;
   p.save_every = a->save_every;
