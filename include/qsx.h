@@ -94,6 +94,18 @@ int qsx_redfield_operators_batched(const double* E, const double* U, int n,
                                    void* stream);
 
 /*
+ * Site-energy shifts of disorder samples start .. start + batch - 1:
+ * out[s][i] = scale * the normals that a RandomState seeded with the array
+ * (seed words, sample index) draws first (the per-sample streams of
+ * Hamiltonian.sample, qspectra/hamiltonian.py:233-274, 552-578).  `seed` is a
+ * host array of nseed < QSX_DISORDER_MAX_KEY words; out [batch][n_sites]
+ * double on the device.
+ */
+#define QSX_DISORDER_MAX_KEY 16
+int qsx_disorder_draws(const uint32_t* seed, int nseed, int64_t start, int64_t batch,
+                       int n_sites, double scale, double* out, void* stream);
+
+/*
  * Rotating-frame Hamiltonians of disorder samples: H[s] = base + diag of
  * offsets[s] ([batch][n_sites]) on rows/columns [off, off + n_sites) of the
  * shared n x n base (the site-energy shifts of Hamiltonian.sample,

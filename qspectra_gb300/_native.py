@@ -154,6 +154,8 @@ _PROTOS = {
                                             _c_vp, _c_vp, _c_vp]),
     'qsx_debye_matsubara_table': (_c_int, [_c_dbl, _c_dbl, _c_int, _c_int, _c_dbl, _c_vp]),
     'qsx_debye_matsubara_table_degree': (_c_int, []),
+    'qsx_disorder_draws': (_c_int, [ctypes.POINTER(ctypes.c_uint32), _c_int, _c_i64, _c_i64,
+                                    _c_int, _c_dbl, _c_vp, _c_vp]),
     'qsx_disordered_hamiltonians': (_c_int, [_c_vp, _c_int, _c_vp, _c_i64, _c_int, _c_int,
                                              _c_vp, _c_vp]),
     'qsx_gemm_batched': (_c_int, [_c_int, _c_int, _c_i64, _c_int, _c_int, _c_int, _c_vp,
@@ -312,6 +314,22 @@ def redfield_operators_w32(E, U, n_sites, off, bath, unit_convert, discard_imag_
         bath.cutoff_freq, matsubara_cutoff, int(discard_imag_corr), unit_convert, _p(G),
         _p(M), _stream()), 'qsx_redfield_operators_w32')
     return G, M
+
+
+DISORDER_MAX_SEED = 15   # QSX_DISORDER_MAX_KEY - 1
+
+
+def disorder_draws(seed, start, batch, n_sites, scale):
+    """(batch, n_sites) float64: scale times the normals of the streams
+    RandomState(seed + [n]), n = start .. start + batch - 1
+    (qsx_disorder_draws); ``seed`` is a list of at most DISORDER_MAX_SEED
+    words."""
+    require_gpu()
+    words = (ctypes.c_uint32 * max(len(seed), 1))(*seed)
+    out = torch.empty((batch, n_sites), dtype=torch.float64, device='cuda')
+    _check(load().qsx_disorder_draws(words, len(seed), start, batch, n_sites, float(scale),
+                                     _p(out), _stream()), 'qsx_disorder_draws')
+    return out
 
 
 def disordered_hamiltonians(base, offsets, off):

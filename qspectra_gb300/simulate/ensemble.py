@@ -11,8 +11,32 @@ import numpy as np
 import torch
 
 from .. import _native
+from ..constants import GAUSSIAN_SD_FWHM
 from ..dynamics.redfield import RedfieldModel
+from ..hamiltonian import ElectronicHamiltonian
 from ..operator_tools import hilbert_subspace_index
+
+
+def disorder_offsets(ham, size, start=0):
+    """``ham.disorder_offsets(size, start)``, drawn on the GPU when the
+    disorder is a plain Gaussian width: there each sample's stream costs a
+    fraction of a microsecond, on the host 88 (a RandomState per sample).
+    The draws are the same to the last bit of a logarithm.  Disorder given as
+    a function, seeds that are not a few 32-bit words (an array seed's own
+    errors included) and classes with draws of their own stay on the host."""
+    base = ham._not_sampled
+    seed = np.atleast_1d(base.random_seed)
+    if (not all(type(h).disorder_offsets is ElectronicHamiltonian.disorder_offsets
+                for h in (ham, base))
+            or type(base)._disorder_for is not ElectronicHamiltonian._disorder_for
+            or type(base)._seed_for is not ElectronicHamiltonian._seed_for
+            or not isinstance(base.disorder, (int, float)) or seed.ndim != 1
+            or seed.dtype.kind not in 'iu' or seed.size > _native.DISORDER_MAX_SEED
+            or (seed.size and (seed.min() < 0 or seed.max() >= 1 << 32))
+            or start < 0 or start + size > 1 << 32 or size < 1):
+        return ham.disorder_offsets(size, start)
+    return _native.disorder_draws([int(w) for w in seed], start, size, ham.n_sites,
+                                  base.disorder * GAUSSIAN_SD_FWHM)
 
 
 class SampleBatch:
@@ -29,7 +53,7 @@ class SampleBatch:
         self.start = int(start)
         ham = model.hamiltonian
         if offsets is None:
-            offsets = ham.disorder_offsets(size, start)
+            offsets = disorder_offsets(ham, self.size, self.start)
         if isinstance(offsets, torch.Tensor):
             self.offsets = offsets.to(device='cuda', dtype=torch.float64)
         else:

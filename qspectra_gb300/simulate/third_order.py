@@ -44,7 +44,7 @@ from ..dynamics.redfield import RedfieldBuild, RedfieldModel
 from ..operator_tools import occupation_table
 from ..dynamics.liouville_space import liouville_subspace_index
 from ..polarization import check_polarizations, isotropic_tensor_4th_order
-from .ensemble import SampleBatch
+from .ensemble import SampleBatch, disorder_offsets
 from .utils import PRECISIONS, step_plan
 
 ENGINE_GEOMETRIES = ('-++', '+-+')
@@ -412,7 +412,7 @@ def third_order_ensemble(model, coherence_time_max, population_times, geometry='
         offsets = np.zeros((1, ham.n_sites))
         count = 1
     else:
-        offsets = ham.disorder_offsets(ensemble_size)
+        offsets = disorder_offsets(ham, ensemble_size)
         count = ensemble_size
         if random_orientations:
             rotations = ham.orientation_rotations(ensemble_size)
