@@ -630,6 +630,19 @@ int qsx_rk4_adjoint_batched(const double* D, int m, int64_t batch, int nsteps,
                             double* gradD, double* grady0, void* stream);
 
 /*
+ * The same gradient from the initial states (complex128 [batch][m],
+ * y0_stride 0 = shared) instead of checkpoints: blocks up to 16 rows and 4095
+ * steps run in blocks of 32 steps on the device, others step by step with a
+ * checkpoint every ck_every steps, which the workspace holds
+ * (qsx_rk4_mean_adjoint_workspace_bytes, 16-byte aligned).  m <= 32.
+ */
+size_t qsx_rk4_mean_adjoint_workspace_bytes(int m, int64_t batch, int nsteps, int ck_every);
+int qsx_rk4_mean_adjoint(const double* D, int m, int64_t batch, int nsteps,
+                         const double* y0, int64_t y0_stride, int ck_every, const double* c,
+                         const double* g, double scale, double* gradD, void* workspace,
+                         size_t workspace_bytes, void* stream);
+
+/*
  * Two-exciton (f) manifold in operator form, for third_order_response
  * (qspectra/simulate/response.py:267-337) at site counts where the dense
  * 'gef' Redfield tensor (qspectra/dynamics/redfield.py:9-74, n^4 entries)

@@ -187,6 +187,10 @@ _PROTOS = {
     'qsx_eigh_large_workspace_bytes': (ctypes.c_size_t, [_c_int, _c_i64]),
     'qsx_eigh_large_batched': (_c_int, [_c_vp, _c_int, _c_i64, _c_vp, _c_vp, _c_vp,
                                         ctypes.c_size_t, _c_vp, _c_vp]),
+    'qsx_rk4_mean_adjoint_workspace_bytes': (ctypes.c_size_t, [_c_int, _c_i64, _c_int, _c_int]),
+    'qsx_rk4_mean_adjoint': (_c_int, [_c_vp, _c_int, _c_i64, _c_int, _c_vp, _c_i64, _c_int,
+                                      _c_vp, _c_vp, _c_dbl, _c_vp, _c_vp, ctypes.c_size_t,
+                                      _c_vp]),
     'qsx_rk4_adjoint_batched': (_c_int, [_c_vp, _c_int, _c_i64, _c_int, _c_vp, _c_int,
                                          _c_int, _c_vp, _c_vp, _c_dbl, _c_vp, _c_vp, _c_vp]),
 }
@@ -1119,6 +1123,27 @@ def rk4_adjoint(D, checkpoints, ck_every, nsteps, c, g, scale, want_y0=False):
                                           float(scale), _p(gradD), _p(gy), _stream()),
            'qsx_rk4_adjoint_batched')
     return (gradD, gy) if want_y0 else gradD
+
+
+def rk4_mean_adjoint(D, y0, ck_every, nsteps, c, g, scale):
+    """rk4_adjoint's gradient w.r.t. D from the initial states y0 ((m,) or
+    (B, m) complex128) instead of checkpoints (qsx_rk4_mean_adjoint)."""
+    require_gpu()
+    _need(D, torch.complex128, 'D', 3)
+    y0 = _need(y0.to(torch.complex128).contiguous(), torch.complex128, 'y0')
+    c = _need(c.to(torch.complex128).contiguous(), torch.complex128, 'c', 1)
+    g = _need(g.to(torch.complex128).contiguous(), torch.complex128, 'g', 1)
+    B, m, _ = D.shape
+    if g.numel() != nsteps + 1 or c.numel() != m or tuple(y0.shape) not in ((m,), (B, m)):
+        raise ValueError('g needs nsteps+1 entries, c m entries and y0 one or B states')
+    lib = load()
+    nbytes = lib.qsx_rk4_mean_adjoint_workspace_bytes(m, B, int(nsteps), int(ck_every))
+    ws = torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=D.device)
+    gradD = torch.empty_like(D)
+    _check(lib.qsx_rk4_mean_adjoint(_p(D), m, B, int(nsteps), _p(y0), m if y0.dim() == 2 else 0,
+                                    int(ck_every), _p(c), _p(g), float(scale), _p(gradD),
+                                    _p(ws), ws.numel(), _stream()), 'qsx_rk4_mean_adjoint')
+    return gradD
 
 
 def eigh_large(H):

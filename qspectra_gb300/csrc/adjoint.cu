@@ -15,7 +15,10 @@
 // forward states are not stored: the caller passes checkpoints every K
 // steps and each segment is recomputed into shared memory before its
 // backward sweep.  One warp per sample, one lane per row (m <= 32), FP64.
+#include <algorithm>
+
 #include "qsx_common.cuh"
+#include "rk4_mean.cuh"
 
 namespace qsx {
 
@@ -29,10 +32,12 @@ struct AdjP {
   int m, nsteps, K, nck;
   int64_t batch;
   double scale;
+  const int* only_if;  // run only when this device word is nonzero (null: always)
 };
 
 __global__ void __launch_bounds__(128) rk4_adjoint_kernel(AdjP p) {
   extern __shared__ __align__(16) unsigned char smraw[];
+  if (p.only_if && *p.only_if == 0) return;
   const int m = p.m, K = p.K;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
@@ -94,10 +99,10 @@ __global__ void __launch_bounds__(128) rk4_adjoint_kernel(AdjP p) {
 
 using namespace qsx;
 
-extern "C" int qsx_rk4_adjoint_batched(const double* D, int m, int64_t batch, int nsteps,
-                                       const double* checkpoints, int ck_every, int nck,
-                                       const double* c, const double* g, double scale,
-                                       double* gradD, double* grady0, void* stream) {
+static int adjoint_stepped(const double* D, int m, int64_t batch, int nsteps,
+                           const double* checkpoints, int ck_every, int nck, const double* c,
+                           const double* g, double scale, double* gradD, double* grady0,
+                           const int* only_if, void* stream) {
   QSX_CHECK_ARG(m >= 1 && m <= 32, "qsx_rk4_adjoint_batched: m=%d outside 1..32", m);
   QSX_CHECK_ARG(batch >= 0 && nsteps >= 0 && ck_every >= 1 && ck_every <= 1024,
                 "qsx_rk4_adjoint_batched: bad batch, step count or checkpoint spacing");
@@ -119,6 +124,7 @@ extern "C" int qsx_rk4_adjoint_batched(const double* D, int m, int64_t batch, in
   p.nck = nck;
   p.batch = batch;
   p.scale = scale;
+  p.only_if = only_if;
   const size_t per_warp = ((size_t)2 * m * m + (size_t)(ck_every + 1) * m) * sizeof(double2);
   int warps = 4;
   while (warps > 1 && per_warp * warps > 96 * 1024) warps >>= 1;
@@ -133,4 +139,67 @@ extern "C" int qsx_rk4_adjoint_batched(const double* D, int m, int64_t batch, in
   rk4_adjoint_kernel<<<grid, 32 * warps, smem, (cudaStream_t)stream>>>(p);
   QSX_LAUNCH_CHECK("qsx_rk4_adjoint_batched");
   return QSX_OK;
+}
+
+extern "C" int qsx_rk4_adjoint_batched(const double* D, int m, int64_t batch, int nsteps,
+                                       const double* checkpoints, int ck_every, int nck,
+                                       const double* c, const double* g, double scale,
+                                       double* gradD, double* grady0, void* stream) {
+  return adjoint_stepped(D, m, batch, nsteps, checkpoints, ck_every, nck, c, g, scale, gradD,
+                         grady0, nullptr, stream);
+}
+
+// checkpoints of the stepped adjoint: y at 0, ck_every, .. below nsteps
+static int64_t checkpoint_count(int nsteps, int ck_every) {
+  return std::max<int64_t>(1, ((int64_t)nsteps + ck_every - 1) / ck_every);
+}
+
+extern "C" size_t qsx_rk4_mean_adjoint_workspace_bytes(int m, int64_t batch, int nsteps,
+                                                       int ck_every) {
+  if (m < 1 || batch < 0 || nsteps < 0 || ck_every < 1) return 0;
+  return 16 + (size_t)batch * checkpoint_count(nsteps, ck_every) * m * sizeof(double2);
+}
+
+extern "C" int qsx_rk4_mean_adjoint(const double* D, int m, int64_t batch, int nsteps,
+                                    const double* y0, int64_t y0_stride, int ck_every,
+                                    const double* c, const double* g, double scale,
+                                    double* gradD, void* workspace, size_t workspace_bytes,
+                                    void* stream) {
+  QSX_CHECK_ARG(m >= 1 && m <= 32 && batch >= 0 && batch <= 0x7fffffffLL && nsteps >= 0 &&
+                    ck_every >= 1,
+                "qsx_rk4_mean_adjoint: bad sizes");
+  if (batch == 0) return QSX_OK;
+  const size_t need = qsx_rk4_mean_adjoint_workspace_bytes(m, batch, nsteps, ck_every);
+  QSX_CHECK_ARG(D && y0 && c && g && gradD && workspace && ((uintptr_t)workspace & 15) == 0,
+                "qsx_rk4_mean_adjoint: null or misaligned pointer");
+  QSX_CHECK_ARG(workspace_bytes >= need,
+                "qsx_rk4_mean_adjoint: workspace of %zu bytes needed (got %zu)", need,
+                workspace_bytes);
+  cudaStream_t s = (cudaStream_t)stream;
+  int* flag = nullptr;
+  if (rk4_mean_adjoint_supported(m, nsteps)) {
+    flag = (int*)workspace;
+    int st = rk4_mean_adjoint_run((const double2*)D, m, batch, nsteps, (const double2*)y0,
+                                  y0_stride, (const double2*)c, (const double2*)g, scale,
+                                  (double2*)gradD, flag, s);
+    if (st) return st;
+  }
+  // step by step from checkpoints: the sizes above, and whatever overflowed
+  const int nck = (int)checkpoint_count(nsteps, ck_every);
+  double* ck = (double*)((char*)workspace + 16);
+  qsx_rk4_args a = {};
+  a.precision = QSX_FP64;
+  a.m = m;
+  a.nsteps = (nck - 1) * ck_every;
+  a.save_every = ck_every;
+  a.batch = batch;
+  a.matrix = D;
+  a.matrix_stride = (int64_t)m * m;
+  a.y0 = y0;
+  a.y0_stride = y0_stride;
+  a.out_state = ck;
+  int st = rk4_stepped_states(&a, flag, s);
+  if (st) return st;
+  return adjoint_stepped(D, m, batch, nsteps, ck, ck_every, nck, c, g, scale, gradD, nullptr,
+                         flag, stream);
 }

@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "qsx_common.cuh"
+#include "rk4_mean.cuh"
 #include "rk4_traj.cuh"
 
 namespace qsx {
@@ -878,8 +879,9 @@ __global__ void __launch_bounds__(1024) rk4_generic(Rk4P p, int mat_in_smem) {
 template <typename P>
 __global__ void __launch_bounds__(256)
     rk4_reduce_kernel(const P* __restrict__ partial, int64_t nslots, int64_t per, double scale,
-                      double2* out) {
+                      double2* out, const int* only_if = nullptr) {
   __shared__ double2 red[8][32];
+  if (only_if && *only_if == 0) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t e = (int64_t)blockIdx.x * 32 + lane;
   double2 acc = make_double2(0.0, 0.0);
@@ -1073,6 +1075,73 @@ static int make_plan(const qsx_rk4_args* a, Plan* pl) {
   return generic_plan(a, pl);
 }
 
+static Rk4P params(const qsx_rk4_args* a) {
+  Rk4P p;
+  p.m = a->m;
+  p.nsteps = a->nsteps;
+  p.save_every = a->save_every;
+  p.nsave = a->nsteps / a->save_every + 1;
+  p.nproj = a->nproj;
+  p.nselect = a->nselect;
+  p.nout = a->nproj > 0 ? a->nproj : a->nselect;
+  p.form = a->form;
+  p.batch = a->batch;
+  p.matrix = a->matrix;
+  p.matrix_stride = a->matrix_stride;
+  p.h = a->h;
+  p.y0 = (const double2*)a->y0;
+  p.y0_stride = a->y0_stride;
+  p.proj = (const double2*)a->proj;
+  p.proj_stride = a->proj_stride;
+  p.select = a->select;
+  p.out_state = (double2*)a->out_state;
+  p.out_proj = (double2*)a->out_proj;
+  p.partial = nullptr;
+  p.partial32 = nullptr;
+  p.status = a->status;
+  p.only_if = nullptr;
+  return p;
+}
+
+// rk4_generic asks for more shared memory than the default limit
+template <typename T>
+static int launch_generic(const Rk4P& p, const Plan& pl, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(rk4_generic<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)pl.smem);
+  if (e != cudaSuccess) return cuda_status(e, "qsx_rk4_batched");
+  rk4_generic<T><<<(unsigned)pl.grid, pl.threads, pl.smem, s>>>(p, pl.mat_in_smem);
+  QSX_LAUNCH_CHECK("qsx_rk4_batched");
+  return QSX_OK;
+}
+
+int rk4_stepped_states(const qsx_rk4_args* a, const int* only_if, cudaStream_t s) {
+  Plan pl;
+  int st = validate(a);
+  if (st == QSX_OK) st = generic_plan(a, &pl);
+  if (st) return st;
+  Rk4P p = params(a);
+  p.only_if = only_if;
+  return launch_generic<double>(p, pl, s);
+}
+
+// The mean of one projection of small blocks, in blocks of steps (rk4_mean.cu):
+// FP64, and the FP32 sizes whose stepped loop is the generic one (its
+// arithmetic is FP64 either way).  Workspace: the stepped loop's partial sums
+// (it runs instead when something overflows), a flag, the blocks' own.
+static int mean_plan(const qsx_rk4_args* a, const Plan& pl, int* grid, size_t* offset,
+                     size_t* bytes) {
+  const int64_t nsave = a->nsteps / a->save_every + 1;
+  *bytes = 0;
+  if (pl.kind != K_GENERIC || !a->out_mean || a->out_state || a->out_proj || a->form != 0 ||
+      a->nproj != 1 || a->variant || a->save_every != 1 || !rk4_mean_supported(a->m, nsave))
+    return QSX_OK;
+  int st = rk4_mean_grid(a->batch, grid);
+  if (st) return st;
+  *offset = (size_t)pl.nslots * nsave * sizeof(double2);
+  *bytes = *offset + 16 + (size_t)*grid * nsave * sizeof(double2);
+  return QSX_OK;
+}
+
 }  // namespace qsx
 
 using namespace qsx;
@@ -1099,7 +1168,11 @@ int qsx_rk4_workspace_bytes(const qsx_rk4_args* a, size_t* bytes) {
   const int64_t nsave = a->nsteps / a->save_every + 1;
   const int64_t nout = a->nproj > 0 ? a->nproj : a->nselect;
   *bytes = (size_t)pl.nslots * nsave * nout * partial_bytes(pl.kind);
-  return QSX_OK;
+  int grid;
+  size_t offset, mean;
+  st = mean_plan(a, pl, &grid, &offset, &mean);
+  *bytes = std::max(*bytes, mean);
+  return st;
 }
 
 int qsx_rk4_batched(const qsx_rk4_args* a, void* stream) {
@@ -1108,8 +1181,7 @@ int qsx_rk4_batched(const qsx_rk4_args* a, void* stream) {
   if (a->batch == 0) return QSX_OK;
   cudaStream_t s = (cudaStream_t)stream;
   Plan pl;
-  Rk4P p;
-  p.only_if = nullptr;
+  Rk4P p = params(a);
   // few samples with every state wanted: by doubling, given the workspace
   TrajPlan tr;
   st = rk4_traj_plan(a, &tr);
@@ -1125,28 +1197,6 @@ int qsx_rk4_batched(const qsx_rk4_args* a, void* stream) {
     st = make_plan(a, &pl);
   }
   if (st) return st;
-  p.m = a->m;
-  p.nsteps = a->nsteps;
-  p.save_every = a->save_every;
-  p.nsave = a->nsteps / a->save_every + 1;
-  p.nproj = a->nproj;
-  p.nselect = a->nselect;
-  p.nout = a->nproj > 0 ? a->nproj : a->nselect;
-  p.form = a->form;
-  p.batch = a->batch;
-  p.matrix = a->matrix;
-  p.matrix_stride = a->matrix_stride;
-  p.h = a->h;
-  p.y0 = (const double2*)a->y0;
-  p.y0_stride = a->y0_stride;
-  p.proj = (const double2*)a->proj;
-  p.proj_stride = a->proj_stride;
-  p.select = a->select;
-  p.out_state = (double2*)a->out_state;
-  p.out_proj = (double2*)a->out_proj;
-  p.partial = nullptr;
-  p.partial32 = nullptr;
-  p.status = a->status;
   const int64_t per = (int64_t)p.nsave * p.nout;
   if (a->out_mean) {
     size_t need = (size_t)pl.nslots * per * partial_bytes(pl.kind);
@@ -1162,6 +1212,21 @@ int qsx_rk4_batched(const qsx_rk4_args* a, void* stream) {
     } else {
       p.partial32 = (float2*)a->workspace;
     }
+  }
+  int grid = 0;
+  size_t offset = 0, mean = 0;
+  st = mean_plan(a, pl, &grid, &offset, &mean);
+  if (st) return st;
+  if (mean && a->workspace_bytes >= mean && ((uintptr_t)a->workspace & 15) == 0) {
+    char* ws = (char*)a->workspace;
+    int* flag = (int*)(ws + offset);
+    double2* sums = (double2*)(ws + offset + 16);
+    st = rk4_mean_run(a, grid, sums, flag, s);
+    if (st) return st;
+    rk4_reduce_kernel<double2><<<(unsigned)((per + 31) / 32), 256, 0, s>>>(
+        sums, grid, per, a->mean_scale, (double2*)a->out_mean);
+    QSX_LAUNCH_CHECK("qsx_rk4_batched mean reduce");
+    p.only_if = flag;   // the stepped loop below, if something was not finite
   }
   switch (pl.kind) {
     case K_SMALL: {
@@ -1202,18 +1267,9 @@ int qsx_rk4_batched(const qsx_rk4_args* a, void* stream) {
       break;
     }
     case K_GENERIC: {
-      cudaError_t e;
-      if (a->precision == QSX_FP32) {
-        e = cudaFuncSetAttribute(rk4_generic<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)pl.smem);
-        if (e != cudaSuccess) return cuda_status(e, "qsx_rk4_batched");
-        rk4_generic<float><<<(unsigned)pl.grid, pl.threads, pl.smem, s>>>(p, pl.mat_in_smem);
-      } else {
-        e = cudaFuncSetAttribute(rk4_generic<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)pl.smem);
-        if (e != cudaSuccess) return cuda_status(e, "qsx_rk4_batched");
-        rk4_generic<double><<<(unsigned)pl.grid, pl.threads, pl.smem, s>>>(p, pl.mat_in_smem);
-      }
+      st = a->precision == QSX_FP32 ? launch_generic<float>(p, pl, s)
+                                    : launch_generic<double>(p, pl, s);
+      if (st) return st;
       break;
     }
   }
@@ -1222,7 +1278,7 @@ int qsx_rk4_batched(const qsx_rk4_args* a, void* stream) {
     const unsigned rg = (unsigned)((per + 31) / 32);
     if (pl.kind == K_GENERIC || pl.kind == K_BLOCK)
       rk4_reduce_kernel<double2><<<rg, 256, 0, s>>>(p.partial, pl.nslots, per, a->mean_scale,
-                                                    (double2*)a->out_mean);
+                                                    (double2*)a->out_mean, p.only_if);
     else
       rk4_reduce_kernel<float2><<<rg, 256, 0, s>>>(p.partial32, pl.nslots, per,
                                                    a->mean_scale, (double2*)a->out_mean);

@@ -14,10 +14,9 @@ the bath reorganisation energy of a Redfield model (redfield.py:9-152).
   derivative), and the operator-form Redfield tensor.
 * The RK4 time loop and its adjoint are hand-written kernels behind
   ``ProjectedMeanRK4``: forward ``qsx_rk4_batched`` (ensemble-mean
-  projection, checkpoints every K steps), backward
-  ``qsx_rk4_adjoint_batched`` (lambda backward under P^H, gradient
-  sum_k lambda_{k+1} y_k^H accumulated per sample, segments recomputed from
-  the checkpoints).
+  projection), backward ``qsx_rk4_mean_adjoint`` (the forward's block states
+  recomputed, then its blocks in reverse; larger blocks step by step, lambda
+  backward under P^H from checkpoints every ``ck_every`` steps).
 * The transform to the frequency grid is ``qsx_dft_batched`` forward and,
   with the roles of time and frequency exchanged, backward.
 """
@@ -140,19 +139,18 @@ class ProjectedMeanRK4(torch.autograd.Function):
         S, m, _ = D.shape
         out = _native.rk4(D, y0, nsteps, 1, proj=c[None], per_sample=False, mean=True,
                           precision=_native.QSX_FP64)
-        nck = max(1, -(-nsteps // ck_every))
-        ck = _native.rk4(D, y0, (nck - 1) * ck_every, ck_every, state=True,
-                         precision=_native.QSX_FP64)['state'] if nck > 1 else \
-            y0.to(torch.complex128).expand(S, 1, m).contiguous()
-        ctx.save_for_backward(D, ck, c)
+        if ck_every < 1:
+            raise ValueError('ck_every must be at least 1')
+        # a copy: the caller may reuse y0's memory before the backward pass
+        ctx.save_for_backward(D, y0.to(torch.complex128).clone(), c)
         ctx.nsteps, ctx.ck_every = nsteps, ck_every
         return out['mean'][:, 0]
 
     @staticmethod
     def backward(ctx, g):
-        D, ck, c = ctx.saved_tensors
-        gradD = _native.rk4_adjoint(D, ck.contiguous(), ctx.ck_every, ctx.nsteps, c,
-                                    g.contiguous(), 1.0 / D.shape[0])
+        D, y0, c = ctx.saved_tensors
+        gradD = _native.rk4_mean_adjoint(D, y0, ctx.ck_every, ctx.nsteps, c, g.contiguous(),
+                                         1.0 / D.shape[0])
         return gradD, None, None, None, None
 
 
