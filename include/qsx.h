@@ -643,6 +643,36 @@ int qsx_rk4_mean_adjoint(const double* D, int m, int64_t batch, int nsteps,
                          size_t workspace_bytes, void* stream);
 
 /*
+ * The differentiable 'eg' generator of absorption fits, FP64, n <= 16 sites
+ * (no reference counterpart; the formulas are those of
+ * qspectra/dynamics/redfield.py:41-104 and qspectra/bath.py:84-102).
+ *
+ * qsx_debye_unit: the one-sided Debye correlation function without its factor
+ * lambda, and its derivative, at count frequencies x (complex128 [count]).
+ * qsx_eg_generator: from H, U double [batch][n][n] and E [batch][n] (its
+ * eigenpairs) L = -(G + i uc H)^T complex128 [batch][n][n]; c0, d0 complex128
+ * [batch][n][n] are the unit correlation function at E_d - E_c and its
+ * derivative, which the adjoint reads.  lam is a device scalar.
+ * qsx_eg_generator_adjoint: cotangent gL of L to gH double [batch][n][n] and
+ * glam [batch] (the cotangent of lam, per sample).
+ * qsx_rk4_step: D = P - I of one RK4 step; qsx_rk4_step_adjoint: cotangent gD
+ * of D to gL.  Cotangents follow PyTorch's convention for complex tensors.
+ */
+int qsx_debye_unit(const double* x, int64_t count, double temperature, double cutoff_freq,
+                   int matsubara_cutoff, double* value, double* derivative, void* stream);
+int qsx_eg_generator(const double* H, const double* E, const double* U, int n, int64_t batch,
+                     const double* lam, double temperature, double cutoff_freq,
+                     int matsubara_cutoff, double unit_convert, double* L, double* c0,
+                     double* d0, void* stream);
+int qsx_eg_generator_adjoint(const double* E, const double* U, int n, int64_t batch,
+                             const double* lam, double unit_convert, const double* c0,
+                             const double* d0, const double* gL, double* gH, double* glam,
+                             void* stream);
+int qsx_rk4_step(const double* L, int n, int64_t batch, double h, double* D, void* stream);
+int qsx_rk4_step_adjoint(const double* L, const double* gD, int n, int64_t batch, double h,
+                         double* gL, void* stream);
+
+/*
  * Two-exciton (f) manifold in operator form, for third_order_response
  * (qspectra/simulate/response.py:267-337) at site counts where the dense
  * 'gef' Redfield tensor (qspectra/dynamics/redfield.py:9-74, n^4 entries)

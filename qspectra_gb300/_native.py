@@ -187,6 +187,13 @@ _PROTOS = {
     'qsx_eigh_large_workspace_bytes': (ctypes.c_size_t, [_c_int, _c_i64]),
     'qsx_eigh_large_batched': (_c_int, [_c_vp, _c_int, _c_i64, _c_vp, _c_vp, _c_vp,
                                         ctypes.c_size_t, _c_vp, _c_vp]),
+    'qsx_debye_unit': (_c_int, [_c_vp, _c_i64, _c_dbl, _c_dbl, _c_int, _c_vp, _c_vp, _c_vp]),
+    'qsx_eg_generator': (_c_int, [_c_vp, _c_vp, _c_vp, _c_int, _c_i64, _c_vp, _c_dbl, _c_dbl,
+                                  _c_int, _c_dbl, _c_vp, _c_vp, _c_vp, _c_vp]),
+    'qsx_eg_generator_adjoint': (_c_int, [_c_vp, _c_vp, _c_int, _c_i64, _c_vp, _c_dbl, _c_vp,
+                                          _c_vp, _c_vp, _c_vp, _c_vp, _c_vp]),
+    'qsx_rk4_step': (_c_int, [_c_vp, _c_int, _c_i64, _c_dbl, _c_vp, _c_vp]),
+    'qsx_rk4_step_adjoint': (_c_int, [_c_vp, _c_vp, _c_int, _c_i64, _c_dbl, _c_vp, _c_vp]),
     'qsx_rk4_mean_adjoint_workspace_bytes': (ctypes.c_size_t, [_c_int, _c_i64, _c_int, _c_int]),
     'qsx_rk4_mean_adjoint': (_c_int, [_c_vp, _c_int, _c_i64, _c_int, _c_vp, _c_i64, _c_int,
                                       _c_vp, _c_vp, _c_dbl, _c_vp, _c_vp, ctypes.c_size_t,
@@ -1144,6 +1151,71 @@ def rk4_mean_adjoint(D, y0, ck_every, nsteps, c, g, scale):
                                     int(ck_every), _p(c), _p(g), float(scale), _p(gradD),
                                     _p(ws), ws.numel(), _stream()), 'qsx_rk4_mean_adjoint')
     return gradD
+
+
+FIT_MAX = 16   # sites of the differentiable generator and RK4 step kernels
+
+
+def debye_unit(x, temperature, cutoff_freq, matsubara_cutoff):
+    """The Debye correlation function over lambda and its derivative at the
+    frequencies x (float64 CUDA, any shape; qsx_debye_unit)."""
+    require_gpu()
+    x = _need(x.contiguous(), torch.float64, 'x')
+    val = torch.empty(x.shape, dtype=torch.complex128, device=x.device)
+    der = torch.empty_like(val)
+    _check(load().qsx_debye_unit(_p(x), x.numel(), float(temperature), float(cutoff_freq),
+                                 int(matsubara_cutoff), _p(val), _p(der), _stream()),
+           'qsx_debye_unit')
+    return val, der
+
+
+def eg_generator(H, E, U, lam, temperature, cutoff_freq, matsubara_cutoff, unit_convert):
+    """L, c0, d0 (S, n, n) complex128 of qsx_eg_generator; lam one float64
+    CUDA element."""
+    require_gpu()
+    S, n, _ = _need(H, torch.float64, 'H', 3).shape
+    L, c0, d0 = (torch.empty((S, n, n), dtype=torch.complex128, device=H.device)
+                 for _ in range(3))
+    _check(load().qsx_eg_generator(_p(H), _p(_need(E, torch.float64, 'E', 2)),
+                                   _p(_need(U, torch.float64, 'U', 3)), n, S,
+                                   _p(_need(lam, torch.float64, 'lam')), float(temperature),
+                                   float(cutoff_freq), int(matsubara_cutoff),
+                                   float(unit_convert), _p(L), _p(c0), _p(d0), _stream()),
+           'qsx_eg_generator')
+    return L, c0, d0
+
+
+def eg_generator_adjoint(E, U, lam, unit_convert, c0, d0, gL):
+    """(gH (S, n, n), glam (S,)) float64 of qsx_eg_generator_adjoint."""
+    require_gpu()
+    S, n, _ = _need(U, torch.float64, 'U', 3).shape
+    gL = _need(gL.to(torch.complex128).contiguous(), torch.complex128, 'gL', 3)
+    gH = torch.empty_like(U)
+    glam = torch.empty(S, dtype=torch.float64, device=U.device)
+    _check(load().qsx_eg_generator_adjoint(_p(E), _p(U), n, S, _p(lam), float(unit_convert),
+                                           _p(c0), _p(d0), _p(gL), _p(gH), _p(glam),
+                                           _stream()), 'qsx_eg_generator_adjoint')
+    return gH, glam
+
+
+def rk4_step(L, h):
+    """D = P - I (S, n, n) complex128 of one RK4 step (qsx_rk4_step)."""
+    require_gpu()
+    S, n, _ = _need(L, torch.complex128, 'L', 3).shape
+    D = torch.empty_like(L)
+    _check(load().qsx_rk4_step(_p(L), n, S, float(h), _p(D), _stream()), 'qsx_rk4_step')
+    return D
+
+
+def rk4_step_adjoint(L, gD, h):
+    """Cotangent of L from the cotangent gD of rk4_step's D."""
+    require_gpu()
+    S, n, _ = _need(L, torch.complex128, 'L', 3).shape
+    gD = _need(gD.to(torch.complex128).contiguous(), torch.complex128, 'gD', 3)
+    gL = torch.empty_like(L)
+    _check(load().qsx_rk4_step_adjoint(_p(L), _p(gD), n, S, float(h), _p(gL), _stream()),
+           'qsx_rk4_step_adjoint')
+    return gL
 
 
 def eigh_large(H):

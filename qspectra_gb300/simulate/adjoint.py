@@ -30,7 +30,10 @@ from ..constants import CM_FS, CM_K
 # ------------------------------------------------------------- Debye bath
 def _debye_unit(x, temperature, cutoff_freq, matsubara_cutoff, chunk=8192):
     """C(x) / lambda and dC/dx / lambda by the reference's truncated sum
-    (bath.py:84-102); x = 0 takes the reference's limit lambda (2T/gamma - i)."""
+    (bath.py:84-102); x = 0 takes the reference's limit lambda (2T/gamma - i).
+    On the GPU one kernel evaluates both (qsx_debye_unit)."""
+    if x.is_cuda and x.dtype == torch.float64:
+        return _native.debye_unit(x, temperature, cutoff_freq, matsubara_cutoff)
     T, gam = float(temperature), float(cutoff_freq)
     flat = x.reshape(-1)
     nu = 2 * np.pi * T * torch.arange(1, matsubara_cutoff, dtype=torch.float64,
@@ -97,6 +100,45 @@ class SymmetricEigh(torch.autograd.Function):
 
 
 # --------------------------------------------------------------- generator
+class EgGenerator(torch.autograd.Function):
+    """Heisenberg 'eg' generators L of rotating-frame Hamiltonians H (S, N, N)
+    and a reorganisation energy, N <= 16: one kernel after the eigensolve and
+    one backward (qsx_eg_generator, qsx_eg_generator_adjoint)."""
+
+    @staticmethod
+    def forward(ctx, H, lam, temperature, cutoff_freq, unit_convert, matsubara_cutoff):
+        H = H.detach().contiguous()
+        E, U = _native.eigh(H, [0, H.shape[-1]])
+        L, c0, d0 = _native.eg_generator(H, E, U, lam.detach(), temperature, cutoff_freq,
+                                         matsubara_cutoff, unit_convert)
+        ctx.save_for_backward(E, U, c0, d0, lam)
+        ctx.unit_convert = unit_convert
+        return L
+
+    @staticmethod
+    def backward(ctx, g):
+        E, U, c0, d0, lam = ctx.saved_tensors
+        gH, glam = _native.eg_generator_adjoint(E, U, lam, ctx.unit_convert, c0, d0, g)
+        return gH, glam.sum().reshape(lam.shape), None, None, None, None
+
+
+class RK4Step(torch.autograd.Function):
+    """D = P - I of one RK4 step of L (S, N, N), N <= 16, one kernel each way."""
+
+    @staticmethod
+    def forward(ctx, L, h):
+        # a copy: the caller may reuse L's memory before the backward pass
+        L = L.detach().clone(memory_format=torch.contiguous_format)
+        ctx.save_for_backward(L)
+        ctx.h = h
+        return _native.rk4_step(L, h)
+
+    @staticmethod
+    def backward(ctx, g):
+        (L,) = ctx.saved_tensors
+        return _native.rk4_step_adjoint(L, g, ctx.h), None
+
+
 def eg_heisenberg_generator(H1, lam, temperature, cutoff_freq, rw_freq, unit_convert,
                             matsubara_cutoff=1000, eigh=None):
     """Heisenberg-picture 'eg' Redfield generator L^T (S, N, N) complex128.
@@ -111,6 +153,11 @@ def eg_heisenberg_generator(H1, lam, temperature, cutoff_freq, rw_freq, unit_con
     N = H1.shape[-1]
     eye = torch.eye(N, dtype=torch.float64, device=H1.device)
     H = H1 - rw_freq * eye
+    if (eigh is None and H.is_cuda and H.dtype == torch.float64 and H.dim() == 3
+            and N <= _native.FIT_MAX and isinstance(lam, torch.Tensor) and lam.is_cuda
+            and lam.dtype == torch.float64 and lam.numel() == 1):
+        return EgGenerator.apply(H, lam, float(temperature), float(cutoff_freq), unit_convert,
+                                 matsubara_cutoff)
     E, U = (eigh or SymmetricEigh.apply)(H)
     x = E[:, None, :] - E[:, :, None]                 # x[c][d] = E_d - E_c
     C = DebyeCorr.apply(x, lam, temperature, cutoff_freq, matsubara_cutoff)
@@ -123,6 +170,9 @@ def eg_heisenberg_generator(H1, lam, temperature, cutoff_freq, rw_freq, unit_con
 
 def rk4_step_minus_identity(L, h):
     """D = P - I, P = sum_{k<=4} (hL)^k / k! (Paterson-Stockmeyer form)."""
+    if (L.is_cuda and L.dtype == torch.complex128 and L.dim() == 3
+            and L.shape[-2] == L.shape[-1] <= _native.FIT_MAX and isinstance(h, (int, float))):
+        return RK4Step.apply(L, h)
     A = h * L
     A2 = A @ A
     return A + 0.5 * A2 + A2 @ (A / 6 + A2 / 24)
