@@ -643,6 +643,20 @@ int qsx_rk4_mean_adjoint(const double* D, int m, int64_t batch, int nsteps,
                          size_t workspace_bytes, void* stream);
 
 /*
+ * FP64 ensemble mean of a Hermitian block in its real form:
+ * out[n][q] (double [nsteps + 1][nsel]) = mean over samples of coordinate
+ * select[q] of x_n, x_{n+1} = x_n + D x_n, D double [batch][m][m] (the output
+ * of qsx_redfield_propagator_hermitian_batched), m = 2^2 .. 8^2, x0 double [m]
+ * shared by the samples.  status: QSX_ERR_NONFINITE when a final state is not
+ * finite, QSX_ERR_INVALID_ARG for a bad select entry.
+ */
+size_t qsx_rk4_real_mean_f64_workspace_bytes(int m, int64_t batch, int nsteps, int nsel);
+int qsx_rk4_real_mean_f64(const double* D, int m, int64_t batch, int nsteps,
+                          const double* x0, const int32_t* select, int nsel, double* out,
+                          void* workspace, size_t workspace_bytes, int32_t* status,
+                          void* stream);
+
+/*
  * The differentiable 'eg' generator of absorption fits, FP64, n <= 16 sites
  * (no reference counterpart; the formulas are those of
  * qspectra/dynamics/redfield.py:41-104 and qspectra/bath.py:84-102).

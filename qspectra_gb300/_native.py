@@ -187,6 +187,10 @@ _PROTOS = {
     'qsx_eigh_large_workspace_bytes': (ctypes.c_size_t, [_c_int, _c_i64]),
     'qsx_eigh_large_batched': (_c_int, [_c_vp, _c_int, _c_i64, _c_vp, _c_vp, _c_vp,
                                         ctypes.c_size_t, _c_vp, _c_vp]),
+    'qsx_rk4_real_mean_f64_workspace_bytes': (ctypes.c_size_t, [_c_int, _c_i64, _c_int,
+                                                                _c_int]),
+    'qsx_rk4_real_mean_f64': (_c_int, [_c_vp, _c_int, _c_i64, _c_int, _c_vp, _c_vp, _c_int,
+                                       _c_vp, _c_vp, ctypes.c_size_t, _c_vp, _c_vp]),
     'qsx_debye_unit': (_c_int, [_c_vp, _c_i64, _c_dbl, _c_dbl, _c_int, _c_vp, _c_vp, _c_vp]),
     'qsx_eg_generator': (_c_int, [_c_vp, _c_vp, _c_vp, _c_int, _c_i64, _c_vp, _c_dbl, _c_dbl,
                                   _c_int, _c_dbl, _c_vp, _c_vp, _c_vp, _c_vp]),
@@ -647,6 +651,29 @@ def redfield_propagator_hermitian(H, G, M, occ, states, unit_convert, h, precisi
         _p(recipe), h, precision, _p(D), _stream()),
         'qsx_redfield_propagator_hermitian_batched')
     return D
+
+
+def rk4_real_mean_f64(D, x0, nsteps, select):
+    """((nsteps + 1, len(select)) float64 ensemble mean of the selected
+    coordinates of x_{n+1} = x_n + D x_n, status word); D (B, m, m) float64,
+    x0 (m,) shared (qsx_rk4_real_mean_f64)."""
+    require_gpu()
+    _need(D, torch.float64, 'D', 3)
+    B, m, _ = D.shape
+    x0 = _need(x0.to(device=D.device, dtype=torch.float64).contiguous(), torch.float64, 'x0', 1)
+    sel_np = np.asarray(select, dtype=np.int64).reshape(-1)
+    if x0.numel() != m or sel_np.size == 0 or sel_np.min() < 0 or sel_np.max() >= m:
+        raise ValueError('x0 needs m entries and select indices must lie in [0, m)')
+    sel = const_tensor(sel_np.astype(np.int32), torch.int32, D.device)
+    lib = load()
+    nbytes = lib.qsx_rk4_real_mean_f64_workspace_bytes(m, B, int(nsteps), sel.numel())
+    ws = torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=D.device)
+    out = torch.empty((nsteps + 1, sel.numel()), dtype=torch.float64, device=D.device)
+    status = torch.zeros(1, dtype=torch.int32, device=D.device)
+    _check(lib.qsx_rk4_real_mean_f64(_p(D), m, B, int(nsteps), _p(x0), _p(sel), sel.numel(),
+                                     _p(out), _p(ws), ws.numel(), _p(status), _stream()),
+           'qsx_rk4_real_mean_f64')
+    return out, status
 
 
 def rk4_block_matrix_real(D, K, select):

@@ -324,10 +324,12 @@ def hermitian_block_size(idx, n_total):
 _TENSOR_CORE_BLOCKS = True
 
 
-def propagate_hermitian_mean(build, idx, nb, h, y0, nsteps, select, events=None, x0=None):
-    """FP32 ensemble mean of the selected components of a Hermitian diagonal
-    block through its real form: real propagator, real K-step blocked matrix
-    (tcgen05 3xTF32 products when the shape allows) and real blocked loop.
+def propagate_hermitian_mean(build, idx, nb, h, y0, nsteps, select, events=None, x0=None,
+                             precision=_native.QSX_FP32):
+    """Ensemble mean of the selected components of a Hermitian diagonal
+    block through its real form: real propagator, then in FP32 the real K-step
+    blocked matrix (tcgen05 3xTF32 products when the shape allows) and real
+    blocked loop, in FP64 the stepped real loop.
     Returns {'mean': (nsteps + 1, len(select)) complex128, 'status'} like
     propagate_selected_mean; when every selected component is a population
     (diagonal), 'mean_real' holds the same values as float64 without the
@@ -338,7 +340,22 @@ def propagate_hermitian_mean(build, idx, nb, h, y0, nsteps, select, events=None,
     a, b = sel % nb, sel // nb
     partner = np.where(a == b, sel, b + nb * a)
     coords = np.unique(np.concatenate([sel, partner]))
-    Dr = build.hermitian_propagator(idx, nb, h)
+    Dr = build.hermitian_propagator(idx, nb, h, precision)
+    if precision == _native.QSX_FP64:
+        if x0 is None:
+            x0 = hermitian_coordinates(y0, nb)
+        if events is not None:
+            e0 = torch.cuda.Event(enable_timing=True)
+            e0.record()
+        xm, status = _native.rk4_real_mean_f64(Dr, x0, nsteps, coords)
+        if events is not None:
+            e1 = torch.cuda.Event(enable_timing=True)
+            e1.record()
+            events.setdefault('dyn', []).append((e0, e1))
+            events['dyn_flops'] = 2.0 * Dr.shape[0] * nsteps * m * m
+            events['dyn_block_k'] = 1
+            events['dyn_variant'] = 'real_f64'
+        return _hermitian_result(xm, status, nb, a, b, coords, sel)
     use_tc = _TENSOR_CORE_BLOCKS and Dr.dtype == torch.float32
     if x0 is None:
         x0 = hermitian_coordinates(y0, nb)
@@ -385,27 +402,38 @@ def propagate_hermitian_mean(build, idx, nb, h, y0, nsteps, select, events=None,
                                * mat.shape[1] * m)
         events['dyn_block_k'] = K
         events['dyn_variant'] = 'real'
+    return _hermitian_result(xm, status, nb, a, b, coords, sel)
+
+
+def _hermitian_result(xm, status, nb, a, b, coords, sel):
+    """The result of propagate_hermitian_mean from its real coordinates."""
     if np.all(a == b) and np.array_equal(coords, sel):
         # populations: the coordinates are the values themselves
         return {'mean_real': xm, 'status': status}
-    full = torch.zeros((xm.shape[0], m), dtype=torch.float64, device=xm.device)
+    full = torch.zeros((xm.shape[0], nb * nb), dtype=torch.float64, device=xm.device)
     full[:, _native.const_tensor(coords, torch.int64, xm.device)] = xm
     y = from_hermitian_coordinates(full, nb)
     return {'mean': y[:, _native.const_tensor(sel, torch.int64, xm.device)], 'status': status}
 
 
-def can_use_hermitian(precision, idx, n_total, y0, nsteps):
-    """Whether the real Hermitian form applies: FP32, a diagonal block of
-    3..8 states, a Hermitian initial state and at least one K > 1."""
-    if not _HERMITIAN or precision != _native.QSX_FP32:
+def can_use_hermitian(precision, idx, n_total, y0, nsteps, site_ops=False):
+    """Whether the real Hermitian form applies: a diagonal block of 3..8
+    states, a Hermitian initial state and, in FP32, at least one K > 1.  FP64
+    takes 2..8 states whose propagator the operators give in real form
+    directly (``site_ops``: non-secular, site basis) and a state that is
+    Hermitian to the bit, so that no part of it is dropped."""
+    fp64 = precision == _native.QSX_FP64
+    if not _HERMITIAN or (fp64 and not site_ops):
         return None
     nb = hermitian_block_size(idx, n_total)
-    if nb is None or not 3 <= nb <= 8:
+    if nb is None or not (2 if fp64 else 3) <= nb <= 8:
         return None
     y = y0.detach().cpu().numpy() if isinstance(y0, torch.Tensor) else np.asarray(y0)
     if y.ndim != 1:
         return None
     rho = y.reshape(nb, nb, order='F')
+    if fp64:
+        return nb if np.array_equal(rho, rho.conj().T) else None
     if np.abs(rho - rho.conj().T).max() > 1e-14 * max(np.abs(rho).max(), 1e-300):
         return None
     m = nb * nb
@@ -532,9 +560,10 @@ def ensemble_populations(model, initial_state, duration, ensemble_size,
         select = [i * nn + i for i in range(nn)]
     y0t = torch.as_tensor(y0, dtype=torch.complex128).cuda()
     n_total = model.hamiltonian.n_states(model.hilbert_subspace)
-    nb = can_use_hermitian(prec, idx, n_total, y0, len(t) - 1)
+    nb = can_use_hermitian(prec, idx, n_total, y0, len(t) - 1, build.site_ops)
     if nb is not None:
-        out = propagate_hermitian_mean(build, idx, nb, dt, y0t, len(t) - 1, select)
+        out = propagate_hermitian_mean(build, idx, nb, dt, y0t, len(t) - 1, select,
+                                       precision=prec)
         if 'mean_real' in out:
             out['mean'] = out['mean_real'].to(torch.complex128)
     else:
@@ -658,13 +687,13 @@ class RedfieldEnsembleWorkload:
             p0 = torch.cuda.Event(enable_timing=True)
             p0.record()
         nb = can_use_hermitian(prec, self.idx_ee, self.n_sites + 1, self.y_dyn_np,
-                               len(self.t_dyn) - 1)
+                               len(self.t_dyn) - 1, build.site_ops)
         if nb is not None:
             if self.x_dyn is None:
                 self.x_dyn = hermitian_coordinates(self.y_dyn, nb).contiguous()
             pop = propagate_hermitian_mean(build, self.idx_ee, nb, self.dt, self.y_dyn,
                                            len(self.t_dyn) - 1, self.select, events,
-                                           x0=self.x_dyn)
+                                           x0=self.x_dyn, precision=prec)
         else:
             D_ee = build.propagator(self.idx_ee, self.dt, prec)
             pop = propagate_selected_mean(D_ee, self.y_dyn, len(self.t_dyn) - 1, self.select,
