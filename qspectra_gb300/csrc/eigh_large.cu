@@ -221,8 +221,10 @@ __global__ void eigh_invit_kernel(const double* __restrict__ de, const double* _
   double tnorm = 0.0;
   for (int i = 0; i < n; ++i)
     tnorm = fmax(tnorm, fabs(d[i]) + fabs(e[i]) + (i ? fabs(e[i - 1]) : 0.0));
-  const double ortol = 1e-3 * tnorm;
-  const double tiny = DBL_EPSILON * fmax(tnorm, DBL_MIN);
+  const double ortol = fmax(1e-3 * tnorm, 1e-100);
+  // (a zero matrix, such as the two-exciton energy of a dimer in its mean
+  // rotating frame, would leave a subnormal whose reciprocal overflows)
+  const double tiny = fmax(DBL_EPSILON * tnorm, 1e-100);
   if (j > 0 && w[j] - w[j - 1] < ortol) return;  // not the first of its cluster
   int jend = j + 1;
   while (jend < n && w[jend] - w[jend - 1] < ortol) ++jend;
@@ -263,7 +265,14 @@ __global__ void eigh_invit_kernel(const double* __restrict__ de, const double* _
       }
     }
     u1[n - 1] = pp == 0.0 ? tiny : pp;
-    for (int i = 0; i < n; ++i) x[i] = 1.0;  // the first solve uses U only
+    // the first solve uses U only.  Later vectors of a cluster start from
+    // scattered signs and sizes: T - lam I may be one and the same for them
+    // (a matrix that is diagonal there), and a start shared with the vectors
+    // they are orthogonalised against would leave nothing
+    for (int i = 0; i < n; ++i) {
+      const unsigned hash = ((unsigned)i * 2654435761u) ^ ((unsigned)jj * 2246822519u);
+      x[i] = jj == j ? 1.0 : 1.0 - (double)((hash * 3266489917u) >> 8) * (2.0 / 16777216.0);
+    }
     for (int it = 0; it < 3; ++it) {
       if (it > 0) {
         for (int i = 0; i < n - 1; ++i) {
