@@ -1098,8 +1098,12 @@ def fe_heisenberg_rk4(Q, Ae, Me, pair_sites, y0, nsteps, h, precision=QSX_FP64,
                                      precision, _p(y0), stride, int(nsteps), float(h),
                                      _p(out), _p(ws), ws.numel(), _p(status), _stream()),
            'qsx_fe_heisenberg_rk4')
-    if check_finite and int(status.item()) & QSX_ERR_NONFINITE:
-        raise IntegratorError('non-finite state in the fe propagation')
+    if check_finite:
+        st = int(status.item())
+        if st & QSX_ERR_CUDA:
+            raise QsxError('fe propagation: a grid barrier timed out')
+        if st & QSX_ERR_NONFINITE:
+            raise IntegratorError('non-finite state in the fe propagation')
     return out
 
 

@@ -16,6 +16,8 @@
 //                            operators of the 'fe' block
 //   qsx_fe_heisenberg_rk4    RK4 on the transposed 'fe' block
 //   qsx_csr_map_batched      sparse dipole super-operator maps between blocks
+#include <algorithm>
+
 #include "qsx_bath.cuh"
 #include "qsx_common.cuh"
 
@@ -125,147 +127,331 @@ __global__ void fe_generator_kernel(const T* __restrict__ M, const double* __res
 // transpose, the Heisenberg-picture generator, is
 //   (L^T X)[:, b] = Q_b^T X[:, b] + sum_c X[:, c] R_p[c][b]  (row p),
 // so column b reads Q_b[q][r] along r: coalesced in the layout Q[s][q][b][r].
-// One CTA per (column b, sample), one thread per row; Q is streamed once per
-// stage (the kernel's HBM traffic), X column b and the row operators sit in
-// shared memory.
 struct FeP {
   int P, N;
   const void* Q;          // [batch][P][N][P] complex (T)
-  const void* Ae;         // [batch][N][N] complex (T)
-  const void* Me;         // [batch][N][N][N] complex (T): Me[i][c][b]
+  const void* R;          // [batch][N b][N site][N c] complex (T), see fe_rows_kernel
   const int* pair_sites;  // [P][2]
   double h;
 };
 
-constexpr int FE_THREADS = 320;
-
+// The row operators by column: R[b][site][c] = conj(Me[site][c][b] - Ae[c][b] / 2)
 template <typename T>
-__global__ void __launch_bounds__(FE_THREADS, sizeof(T) == 4 ? 4 : 2)
-    fe_stage_kernel(FeP p, int stage, const typename cplx<T>::type* in,
-                    typename cplx<T>::type* yh, typename cplx<T>::type* yl,
-                    typename cplx<T>::type* acc, typename cplx<T>::type* next) {
-  using C = typename cplx<T>::type;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int P = p.P, N = p.N;
-  const int b = blockIdx.x;
-  const int64_t s = blockIdx.y;
-  // shared: column b of X (the column term) and the row operators for
-  // column b; each thread reads its own row of X from global memory
-  C* sxb = (C*)smraw;          // [P]
-  C* sR = sxb + P;             // [N][N]: conj(Me[i][c][b] - Ae[c][b] / 2)
-  const int64_t per = (int64_t)P * N;
-  const C* x = in + s * per;
-  for (int i = threadIdx.x; i < P; i += blockDim.x) sxb[i] = x[(int64_t)b * P + i];
-  const C* me = (const C*)p.Me + s * (int64_t)N * N * N;
-  const C* ae = (const C*)p.Ae + s * (int64_t)N * N;
-  for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
-    const int site = i / N, c = i % N;
-    const C m = me[((int64_t)site * N + c) * N + b];
-    const C a = ae[(int64_t)c * N + b];
-    sR[i] = cmk(m.x - (T)0.5 * a.x, -(m.y - (T)0.5 * a.y));
+__global__ void fe_rows_kernel(const typename cplx<T>::type* __restrict__ Me,
+                               const typename cplx<T>::type* __restrict__ Ae, int N, int64_t batch,
+                               typename cplx<T>::type* __restrict__ R) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nn = (int64_t)N * N;
+  if (e >= batch * nn * N) return;
+  const int64_t s = e / (nn * N);
+  const int b = (int)(e / nn % N), site = (int)(e / N % N), c = (int)(e % N);
+  const typename cplx<T>::type m = Me[(s * N + site) * nn + (int64_t)c * N + b];
+  const typename cplx<T>::type a = Ae[s * nn + (int64_t)c * N + b];
+  R[e] = cmk(m.x - (T)0.5 * a.x, -(m.y - (T)0.5 * a.y));
+}
+
+// V values of one load: V = 2 takes two complex64 at once (even P keeps them
+// on 16 bytes), V = 1 one complex value
+template <typename T, int V> struct FeVec;
+template <> struct FeVec<float, 2> { using type = float4; };
+template <> struct FeVec<float, 1> { using type = float2; };
+template <> struct FeVec<double, 1> { using type = double2; };
+
+__device__ __forceinline__ void fe_mac(float2 (&k)[2], float4 q, float2 x) {
+  cfma(k[0], make_float2(q.x, q.y), x);
+  cfma(k[1], make_float2(q.z, q.w), x);
+}
+__device__ __forceinline__ void fe_mac(float2 (&k)[1], float2 q, float2 x) { cfma(k[0], q, x); }
+__device__ __forceinline__ void fe_mac(double2 (&k)[1], double2 q, double2 x) { cfma(k[0], q, x); }
+
+// One cooperative kernel runs the loop of all samples, a group of them at a
+// time: Q is read once a stage, so the bound is its traffic, and a group is as
+// many samples as leave Q in the L2 through all their stages (7 of 24 sites,
+// 102 MB).  A launch a stage over all 32 samples streamed Q from HBM at 5.0
+// TB/s, 93 us; 72 us in groups.  (One CTA a column, a launch a stage, 113 us.
+// Two or four independent teams of half- or quarter-size CTAs, one's barrier
+// behind the other's loads: 78 and 100 us, their items too few to come out
+// even.)
+//
+// Work: an item is a tile of rows of one column; four warps share it, each a
+// quarter of the sum over q with eight 16-byte loads a lane in flight, and
+// add up through shared memory.  Eight items run in a CTA, one CTA an SM; the
+// plan picks the tile so that the items come out even over the SMs.
+//
+// The states cross between SMs once a stage: they are read past the L1
+// (ld.global.cg), written, and fenced before the barrier.  Waits are bounded;
+// a barrier that never fills sets QSX_ERR_CUDA and everyone leaves.
+constexpr int FE_ITEM_WARPS = 4;
+constexpr int FE_ITEMS = 8;   // at most: fewer where their shared memory does not fit
+constexpr int FE_THREADS = 32 * FE_ITEM_WARPS * FE_ITEMS;
+
+struct FeLoop {
+  int64_t batch, y0_stride;
+  int group, ntile, tile, nsteps;   // tile: rows of an item, a multiple of V
+  const double2* y0;
+  void *yh, *yl, *acc, *s0, *s1;    // [group][P N] complex (T)
+  double2* out;
+  int* status;
+  unsigned* barrier;                // zeroed: arrivals, then the abort word
+};
+
+// All CTAs of the grid; false when the wait ran out or somebody's did.
+__device__ __forceinline__ bool fe_grid_barrier(unsigned* bar, unsigned target, int* status) {
+  __shared__ int good;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    bool done = false;
+    for (int i = 0; i < (1 << 24); ++i) {
+      unsigned seen;
+      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+      if ((int)(seen - target) >= 0) {
+        done = true;
+        break;
+      }
+      if ((i & 255) == 255 && *(volatile unsigned*)(bar + 1)) break;
+    }
+    if (!done) {
+      atomicExch(bar + 1, 1u);
+      if (status) atomicOr(status, QSX_ERR_CUDA);
+    }
+    good = done;
   }
   __syncthreads();
-  for (int row = threadIdx.x; row < P; row += blockDim.x) {
-  const C* __restrict__ qcol = (const C*)p.Q + (s * P * N + b) * (int64_t)P + row;
-  const int64_t qstride = (int64_t)N * P;
-  C k0 = cmk((T)0, (T)0), k1 = k0, k2 = k0, k3 = k0;
-  // column term sum_q Q_b[q][row] X[q][b], software-pipelined: the next
-  // U rows of Q are in flight while the current U are consumed
-  constexpr int U = 4;
-  C a[U], nx[U];
-  int q = 0;
-  if (P >= U) {
+  return good;
+}
+
+template <typename T, int V>
+__global__ void __launch_bounds__(FE_THREADS, 1) fe_loop_kernel(FeP p, FeLoop l) {
+  using C = typename cplx<T>::type;
+  using L = typename FeVec<T, V>::type;
+  constexpr bool SPLIT = sizeof(T) == 4;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int P = p.P, N = p.N, per = P * N;
+  const int it = threadIdx.x / (32 * FE_ITEM_WARPS), tid = threadIdx.x % (32 * FE_ITEM_WARPS);
+  const int lane = tid & 31, w = tid >> 5;
+  // this item's column of the stage input, row operators and partial sums
+  C* sxb = (C*)smraw + (size_t)it * (P + N * N + FE_ITEM_WARPS * 32 * V);
+  C* sR = sxb + P;
+  C* part = sR + N * N;
+  auto item_sync = [&] {
+    asm volatile("bar.sync %0, %1;" ::"r"(it + 1), "r"(32 * FE_ITEM_WARPS) : "memory");
+  };
+  C *yh = (C*)l.yh, *yl = (C*)l.yl, *acc = (C*)l.acc, *s0 = (C*)l.s0, *s1 = (C*)l.s1;
+  const int ctas = gridDim.x;
+  const T h = (T)p.h, s6 = h / (T)6;
+  unsigned target = 0;
+  bool ok = true;
+  const int64_t tid_all = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t threads_all = (int64_t)ctas * blockDim.x;
+  const int places = blockDim.x / (32 * FE_ITEM_WARPS);
+  for (int64_t g0 = 0; g0 < l.batch; g0 += l.group) {
+    const int live = (int)min((int64_t)l.group, l.batch - g0);
+    for (int64_t e = tid_all; e < (int64_t)live * per; e += threads_all) {
+      const int64_t s = g0 + e / per, r = e % per;
+      const double2 v = l.y0[s * l.y0_stride + r];
+      const C hi = cmk((T)v.x, (T)v.y);
+      yh[e] = hi;
+      if (SPLIT) yl[e] = cmk((T)(v.x - (double)hi.x), (T)(v.y - (double)hi.y));
+      l.out[s * (l.nsteps + 1) * (int64_t)per + r] = v;
+    }
+    target += ctas;
+    if (!fe_grid_barrier(l.barrier, target, l.status)) return;
+    const int items = live * N * l.ntile;
+    for (int step = 1; step <= l.nsteps; ++step) {
+#pragma unroll 1
+      for (int stage = 0; stage < 4; ++stage) {
+        const C* in = stage == 0 ? yh : (stage & 1) ? s0 : s1;
+        C* next = (stage & 1) ? s1 : s0;
+        for (int i = blockIdx.x + it * ctas; i < items; i += places * ctas) {
+          const int col = i / l.ntile, row0 = i % l.ntile * l.tile;
+          const int sl = col / N, b = col % N;
+          const int64_t s = g0 + sl;
+          const C* x = in + (int64_t)sl * per;
+          const C* gr = (const C*)p.R + (s * N + b) * (int64_t)N * N;
+          for (int e = tid; e < P; e += 32 * FE_ITEM_WARPS) sxb[e] = __ldcg(x + (int64_t)b * P + e);
+          for (int e = tid; e < N * N; e += 32 * FE_ITEM_WARPS) sR[e] = __ldcg(gr + e);
+          item_sync();
+          // this warp's part of the column term sum_q Q_b[q][row] X[q][b]
+          const int row = row0 + V * lane;
+          const bool active = V * lane < l.tile && row < P;   // V = 2: P and the tile are even
+          const int q0 = P * w / FE_ITEM_WARPS, q1 = P * (w + 1) / FE_ITEM_WARPS;
+          C k[V];
 #pragma unroll
-    for (int t = 0; t < U; ++t) a[t] = __ldg(qcol + (int64_t)t * qstride);
-    for (; q + 2 * U <= P; q += U) {
+          for (int v = 0; v < V; ++v) k[v] = cmk((T)0, (T)0);
+          if (active) {
+            const C* qcol = (const C*)p.Q + (s * P * N + b) * (int64_t)P + row;
+            constexpr int U = 8;
+            int q = q0;
+            for (; q + U <= q1; q += U) {
+              L a[U];
 #pragma unroll
-      for (int t = 0; t < U; ++t) nx[t] = __ldg(qcol + (int64_t)(q + U + t) * qstride);
+              for (int t = 0; t < U; ++t)
+                a[t] = __ldcg(reinterpret_cast<const L*>(qcol + (int64_t)(q + t) * per));
 #pragma unroll
-      for (int t = 0; t < U; t += 4) {
-        cfma(k0, a[t], sxb[q + t]);
-        cfma(k1, a[t + 1], sxb[q + t + 1]);
-        cfma(k2, a[t + 2], sxb[q + t + 2]);
-        cfma(k3, a[t + 3], sxb[q + t + 3]);
+              for (int t = 0; t < U; ++t) fe_mac(k, a[t], sxb[q + t]);
+            }
+            for (; q < q1; ++q)
+              fe_mac(k, __ldcg(reinterpret_cast<const L*>(qcol + (int64_t)q * per)), sxb[q]);
+            // and of the row term sum_c X[row][c] (T_k + T_l)[c]
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              const int kk = p.pair_sites[2 * (row + v)], ll = p.pair_sites[2 * (row + v) + 1];
+              for (int c = w; c < N; c += FE_ITEM_WARPS) {
+                const C ra = sR[kk * N + c], rb = sR[ll * N + c];
+                cfma(k[v], __ldcg(x + (int64_t)c * P + row + v), cmk(ra.x + rb.x, ra.y + rb.y));
+              }
+            }
+          }
+#pragma unroll
+          for (int v = 0; v < V; ++v) part[w * 32 * V + V * lane + v] = k[v];
+          item_sync();
+          if (tid < l.tile && row0 + tid < P) {
+            C kk = part[tid];
+#pragma unroll
+            for (int q = 1; q < FE_ITEM_WARPS; ++q) kk = cadd2(kk, part[q * 32 * V + tid]);
+            const int r = b * P + row0 + tid;
+            const int64_t idx = (int64_t)sl * per + r;
+            const C y = __ldcg(yh + idx);
+            if (stage == 0) {
+              acc[idx] = kk;
+              next[idx] = cmk(y.x + (T)0.5 * h * kk.x, y.y + (T)0.5 * h * kk.y);
+            } else if (stage < 3) {
+              const C a0 = __ldcg(acc + idx);
+              acc[idx] = cmk(a0.x + (T)2 * kk.x, a0.y + (T)2 * kk.y);
+              const T cst = stage == 1 ? (T)0.5 * h : h;
+              next[idx] = cmk(y.x + cst * kk.x, y.y + cst * kk.y);
+            } else {
+              const C a0 = __ldcg(acc + idx);
+              const T ix = s6 * (a0.x + kk.x), iy = s6 * (a0.y + kk.y);
+              double2 o;
+              if constexpr (SPLIT) {
+                // split-word state: hi + lo with a TwoSum update
+                const C lo = __ldcg(yl + idx);
+                float hx = y.x, lx = lo.x, hy = y.y, ly = lo.y;
+                dd_add(hx, lx, ix);
+                dd_add(hy, ly, iy);
+                yh[idx] = cmk(hx, hy);
+                yl[idx] = cmk(lx, ly);
+                o = make_double2((double)hx + (double)lx, (double)hy + (double)ly);
+              } else {
+                o = cmk(y.x + ix, y.y + iy);
+                yh[idx] = o;
+              }
+              ok = ok && finite2(o);
+              l.out[(s * (l.nsteps + 1) + step) * (int64_t)per + r] = o;
+            }
+          }
+        }
+        target += ctas;
+        if (!fe_grid_barrier(l.barrier, target, l.status)) return;
       }
-#pragma unroll
-      for (int t = 0; t < U; ++t) a[t] = nx[t];
-    }
-#pragma unroll
-    for (int t = 0; t < U; t += 4) {
-      cfma(k0, a[t], sxb[q + t]);
-      cfma(k1, a[t + 1], sxb[q + t + 1]);
-      cfma(k2, a[t + 2], sxb[q + t + 2]);
-      cfma(k3, a[t + 3], sxb[q + t + 3]);
-    }
-    q += U;
-  }
-  for (; q < P; ++q) cfma(k0, __ldg(qcol + (int64_t)q * qstride), sxb[q]);
-  // row term sum_c X[row][c] (T_k + T_l)[c]
-  const int kk = p.pair_sites[2 * row], ll = p.pair_sites[2 * row + 1];
-  const C* xr = x + row;
-  for (int c = 0; c < N; ++c) {
-    const C ra = sR[kk * N + c], rb = sR[ll * N + c];
-    cfma(k1, xr[(int64_t)c * P], cmk(ra.x + rb.x, ra.y + rb.y));
-  }
-  const C k = cmk(k0.x + k1.x + k2.x + k3.x, k0.y + k1.y + k2.y + k3.y);
-  const int64_t idx = s * per + (int64_t)b * P + row;
-  const T h = (T)p.h;
-  if (stage == 0) {
-    acc[idx] = k;
-    const C y = yh[idx];
-    next[idx] = cmk(y.x + (T)0.5 * h * k.x, y.y + (T)0.5 * h * k.y);
-  } else if (stage < 3) {
-    const C a0 = acc[idx];
-    acc[idx] = cmk(a0.x + (T)2 * k.x, a0.y + (T)2 * k.y);
-    const C y = yh[idx];
-    const T cst = stage == 1 ? (T)0.5 * h : h;
-    next[idx] = cmk(y.x + cst * k.x, y.y + cst * k.y);
-  } else {
-    const C a0 = acc[idx];
-    const T s6 = h / (T)6;
-    const T ix = s6 * (a0.x + k.x), iy = s6 * (a0.y + k.y);
-    const C y = yh[idx];
-    if (yl) {
-      // split-word state: hi + lo with a TwoSum update
-      const C l = yl[idx];
-      float hx = (float)y.x, lx = (float)l.x, hy = (float)y.y, ly = (float)l.y;
-      dd_add(hx, lx, (float)ix);
-      dd_add(hy, ly, (float)iy);
-      yh[idx] = cmk((T)hx, (T)hy);
-      yl[idx] = cmk((T)lx, (T)ly);
-    } else {
-      yh[idx] = cmk(y.x + ix, y.y + iy);
     }
   }
-  }
+  if (!ok && l.status) atomicOr(l.status, QSX_ERR_NONFINITE);
 }
 
-template <typename T>
-__global__ void fe_init_kernel(const double2* __restrict__ y0, int64_t y0_stride, int64_t per,
-                               int64_t batch, typename cplx<T>::type* yh,
-                               typename cplx<T>::type* yl) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= per * batch) return;
-  const double2 v = y0[(i / per) * y0_stride + i % per];
-  yh[i] = cmk((T)v.x, (T)v.y);
-  if (yl) yl[i] = cmk((T)(v.x - (double)(T)v.x), (T)(v.y - (double)(T)v.y));
-}
+// The whole loop of samples whose Q fits one CTA's shared memory, one launch
+// and one CTA a sample: thread e owns the elements e, e + 256, .. of X, its
+// state and stage sums in registers, the stage inputs in shared memory.  For
+// these sizes a stage is shorter than its launch: 4 sites, one FP64 sample,
+// 99 steps were 496 launches, 2.2 ms on the device and more between them.
+constexpr int FE_CTA = 256;
+constexpr int FE_EPT = 2;   // elements a thread
 
 template <typename T>
-__global__ void fe_save_kernel(const typename cplx<T>::type* __restrict__ yh,
-                               const typename cplx<T>::type* __restrict__ yl, int64_t per,
-                               int64_t batch, int k, int nsave, double2* __restrict__ out,
-                               int* status) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= per * batch) return;
-  const int64_t s = i / per, e = i % per;
-  double vx = (double)yh[i].x, vy = (double)yh[i].y;
-  if (yl) {
-    vx += (double)yl[i].x;
-    vy += (double)yl[i].y;
+__global__ void __launch_bounds__(FE_CTA)
+    fe_cta_kernel(FeP p, const double2* __restrict__ y0, int64_t y0_stride, int nsteps,
+                  double2* __restrict__ out, int* status) {
+  using C = typename cplx<T>::type;
+  constexpr bool SPLIT = sizeof(T) == 4;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int P = p.P, N = p.N, per = P * N;
+  C* sQ = (C*)smraw;               // [P][N][P]
+  C* sR = sQ + (size_t)per * P;    // [N b][N site][N c]
+  C* sx = sR + (size_t)N * N * N;  // [2][P N] stage input
+  const int64_t s = blockIdx.x;
+  for (int i = threadIdx.x; i < per * P; i += FE_CTA) sQ[i] = ((const C*)p.Q)[s * per * P + i];
+  for (int i = threadIdx.x; i < N * N * N; i += FE_CTA)
+    sR[i] = ((const C*)p.R)[s * (int64_t)N * N * N + i];
+  C yh[FE_EPT], yl[FE_EPT], ac[FE_EPT];
+  int row[FE_EPT], col[FE_EPT], ka[FE_EPT], kb[FE_EPT];
+  double2* o = out + s * (nsteps + 1) * (int64_t)per;
+#pragma unroll
+  for (int i = 0; i < FE_EPT; ++i) {
+    const int e = threadIdx.x + i * FE_CTA;
+    const bool live = e < per;
+    const double2 v = live ? y0[s * y0_stride + e] : make_double2(0.0, 0.0);
+    yh[i] = cmk((T)v.x, (T)v.y);
+    yl[i] = SPLIT ? cmk((T)(v.x - (double)yh[i].x), (T)(v.y - (double)yh[i].y))
+                  : cmk((T)0, (T)0);
+    ac[i] = cmk((T)0, (T)0);
+    row[i] = live ? e % P : 0;
+    col[i] = live ? e / P : 0;
+    ka[i] = live ? p.pair_sites[2 * row[i]] : 0;
+    kb[i] = live ? p.pair_sites[2 * row[i] + 1] : 0;
+    if (live) {
+      sx[e] = yh[i];
+      o[e] = make_double2((double)yh[i].x + (double)yl[i].x, (double)yh[i].y + (double)yl[i].y);
+    }
   }
-  if (status && !(isfinite(vx) && isfinite(vy))) atomicOr(status, QSX_ERR_NONFINITE);
-  out[(s * nsave + k) * per + e] = make_double2(vx, vy);
+  __syncthreads();
+  const T h = (T)p.h, s6 = h / (T)6;
+  bool ok = true;
+  int cur = 0;
+  for (int step = 1; step <= nsteps; ++step) {
+#pragma unroll 1
+    for (int stage = 0; stage < 4; ++stage, cur ^= 1) {
+      const C* in = sx + cur * per;
+      C* nx = sx + (cur ^ 1) * per;
+#pragma unroll
+      for (int i = 0; i < FE_EPT; ++i) {
+        const int e = threadIdx.x + i * FE_CTA;
+        if (e >= per) break;
+        const C* q = sQ + e;              // Q[q][col][row] at q * per + e
+        const C* xb = in + col[i] * P;
+        C k0 = cmk((T)0, (T)0), k1 = k0;
+        int j = 0;
+        for (; j + 1 < P; j += 2) {
+          cfma(k0, q[(size_t)j * per], xb[j]);
+          cfma(k1, q[(size_t)(j + 1) * per], xb[j + 1]);
+        }
+        if (j < P) cfma(k0, q[(size_t)j * per], xb[j]);
+        const C* ra = sR + (col[i] * N + ka[i]) * N;
+        const C* rb = sR + (col[i] * N + kb[i]) * N;
+        for (int c = 0; c < N; ++c)
+          cfma(k1, in[c * P + row[i]], cmk(ra[c].x + rb[c].x, ra[c].y + rb[c].y));
+        const C k = cadd2(k0, k1);
+        if (stage == 0) {
+          ac[i] = k;
+        } else if (stage < 3) {
+          ac[i] = cmk(ac[i].x + (T)2 * k.x, ac[i].y + (T)2 * k.y);
+        } else {
+          const T ix = s6 * (ac[i].x + k.x), iy = s6 * (ac[i].y + k.y);
+          if (SPLIT) {
+            float hx = (float)yh[i].x, lx = (float)yl[i].x, hy = (float)yh[i].y,
+                  ly = (float)yl[i].y;
+            dd_add(hx, lx, (float)ix);
+            dd_add(hy, ly, (float)iy);
+            yh[i] = cmk((T)hx, (T)hy);
+            yl[i] = cmk((T)lx, (T)ly);
+          } else {
+            yh[i] = cmk(yh[i].x + ix, yh[i].y + iy);
+          }
+        }
+        const T cst = stage < 2 ? (T)0.5 * h : h;
+        nx[e] = stage < 3 ? cmk(yh[i].x + cst * k.x, yh[i].y + cst * k.y) : yh[i];
+        if (stage == 3) {
+          const double2 v = make_double2((double)yh[i].x + (double)yl[i].x,
+                                         (double)yh[i].y + (double)yl[i].y);
+          ok = ok && finite2(v);
+          o[(int64_t)step * per + e] = v;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  if (!ok && status) atomicOr(status, QSX_ERR_NONFINITE);
 }
 
 // ------------------------------------------------------------------ CSR map
@@ -355,7 +541,7 @@ extern "C" size_t qsx_fe_heisenberg_workspace_bytes(int P, int N, int64_t batch,
   if (P < 1 || N < 1 || batch < 0) return 0;
   const size_t cs = precision == QSX_FP32 ? sizeof(float2) : sizeof(double2);
   const size_t n = (size_t)P * N * (size_t)batch;
-  return (precision == QSX_FP32 ? 5 : 4) * n * cs;
+  return 16 + ((precision == QSX_FP32 ? 5 : 4) * n + (size_t)N * N * N * (size_t)batch) * cs;
 }
 
 extern "C" int qsx_fe_heisenberg_rk4(const void* Q, const void* Ae, const void* Me,
@@ -381,40 +567,95 @@ extern "C" int qsx_fe_heisenberg_rk4(const void* Q, const void* Ae, const void* 
   p.P = P;
   p.N = N;
   p.Q = Q;
-  p.Ae = Ae;
-  p.Me = Me;
   p.pair_sites = pair_sites;
   p.h = h;
   const int64_t per = (int64_t)P * N;
   const int64_t n = per * batch;
-  const dim3 grid((unsigned)N, (unsigned)batch);
-  const int threads = P >= FE_THREADS ? FE_THREADS : ((P + 31) / 32) * 32;
-  const unsigned eg = (unsigned)((n + 255) / 256);
+  int dev = 0, sms = 0, l2 = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
+  if (e != cudaSuccess) return cuda_status(e, "qsx_fe_heisenberg_rk4");
   auto run = [&](auto tag) -> int {
     using T = decltype(tag);
     using C = typename cplx<T>::type;
-    C* yh = (C*)workspace;
+    unsigned* barrier = (unsigned*)workspace;
+    C* yh = (C*)((char*)workspace + 16);
     C* yl = sizeof(T) == 4 ? yh + n : nullptr;
     C* acc = yh + (sizeof(T) == 4 ? 2 : 1) * n;
     C* s0 = acc + n;
     C* s1 = s0 + n;
-    const size_t smem = ((size_t)P + (size_t)N * N) * sizeof(C);
-    QSX_CHECK_ARG(smem <= 227 * 1024,
-                  "qsx_fe_heisenberg_rk4: %zu bytes of column state exceed shared memory", smem);
-    cudaError_t e = cudaFuncSetAttribute(fe_stage_kernel<T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_status(e, "qsx_fe_heisenberg_rk4");
-    fe_init_kernel<T><<<eg, 256, 0, s>>>((const double2*)y0, y0_stride, per, batch, yh, yl);
-    fe_save_kernel<T><<<eg, 256, 0, s>>>(yh, yl, per, batch, 0, nsteps + 1, (double2*)out,
-                                        status);
-    for (int step = 1; step <= nsteps; ++step) {
-      fe_stage_kernel<T><<<grid, threads, smem, s>>>(p, 0, yh, yh, yl, acc, s0);
-      fe_stage_kernel<T><<<grid, threads, smem, s>>>(p, 1, s0, yh, yl, acc, s1);
-      fe_stage_kernel<T><<<grid, threads, smem, s>>>(p, 2, s1, yh, yl, acc, s0);
-      fe_stage_kernel<T><<<grid, threads, smem, s>>>(p, 3, s0, yh, yl, acc, nullptr);
-      fe_save_kernel<T><<<eg, 256, 0, s>>>(yh, yl, per, batch, step, nsteps + 1,
-                                          (double2*)out, status);
+    C* R = s1 + n;
+    p.R = R;
+    const int64_t rows = batch * (int64_t)N * N * N;
+    fe_rows_kernel<T><<<(unsigned)((rows + 255) / 256), 256, 0, s>>>((const C*)Me, (const C*)Ae,
+                                                                     N, batch, R);
+    // One CTA a sample while Q fits beside the state, and while its stage
+    // (multiply-adds at an SM's rate: 128 a clock in FP32, 2 in FP64, from
+    // shared memory a quarter of the FP32 rate) costs less than the 6 us that
+    // a launched stage takes at least
+    const size_t cta = ((size_t)per * P + (size_t)N * N * N + 2 * (size_t)per) * sizeof(C);
+    const double fma = 4.0 * (double)per * (P + 2 * N);
+    const double stage_us = fma / (sizeof(T) == 4 ? 32.0 : 2.0) / 1900.0 *
+                            (double)((batch + sms - 1) / sms);
+    if (per <= FE_CTA * FE_EPT && cta <= 200 * 1024 && stage_us < 6.0) {
+      e = cudaFuncSetAttribute(fe_cta_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)cta);
+      if (e != cudaSuccess) return cuda_status(e, "qsx_fe_heisenberg_rk4");
+      fe_cta_kernel<T><<<(unsigned)batch, FE_CTA, cta, s>>>(p, (const double2*)y0, y0_stride,
+                                                          nsteps, (double2*)out, status);
+      QSX_LAUNCH_CHECK("qsx_fe_heisenberg_rk4");
+      return QSX_OK;
     }
+    constexpr int V2 = sizeof(T) == 4 ? 2 : 1;
+    const bool wide = P % 2 == 0 && ((uintptr_t)Q & 15) == 0;
+    const int V = wide ? V2 : 1;
+    auto kern = wide ? fe_loop_kernel<T, V2> : fe_loop_kernel<T, 1>;
+    FeLoop l;
+    // samples whose Q stays in the L2 (a fifth is left for the states), the
+    // groups equal
+    const double sample = (double)per * P * sizeof(C);
+    const int64_t fit = std::max<int64_t>(1, (int64_t)(0.8 * l2 / sample));
+    const int64_t groups = (batch + fit - 1) / fit;
+    l.group = (int)((batch + groups - 1) / groups);
+    const size_t item = ((size_t)P + (size_t)N * N + FE_ITEM_WARPS * 32 * V) * sizeof(C);
+    QSX_CHECK_ARG(item <= 220 * 1024,
+                  "qsx_fe_heisenberg_rk4: %zu bytes of column state exceed shared memory", item);
+    const int places = (int)std::min<size_t>(FE_ITEMS, 220 * 1024 / item);
+    // rows of an item: the fewest rows that one place works through in a stage
+    int64_t best = INT64_MAX;
+    for (int nt = (P + 32 * V - 1) / (32 * V); nt <= (P + 7) / 8; ++nt) {
+      const int tile = ((P + nt - 1) / nt + V - 1) / V * V;
+      const int64_t items = (int64_t)l.group * N * ((P + tile - 1) / tile);
+      const int64_t all = (int64_t)places * sms, cost = (items + all - 1) / all * tile;
+      if (cost < best) {
+        best = cost;
+        l.tile = tile;
+        l.ntile = (P + tile - 1) / tile;
+      }
+    }
+    l.batch = batch;
+    l.y0 = (const double2*)y0;
+    l.y0_stride = y0_stride;
+    l.nsteps = nsteps;
+    l.yh = yh;
+    l.yl = yl;
+    l.acc = acc;
+    l.s0 = s0;
+    l.s1 = s1;
+    l.out = (double2*)out;
+    l.status = status;
+    l.barrier = barrier;
+    const size_t smem = places * item;
+    e = cudaMemsetAsync(barrier, 0, 16, s);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int grid = (int)std::min<int64_t>(sms, (int64_t)l.group * N * l.ntile);
+    void* args[] = {&p, &l};
+    if (e == cudaSuccess)
+      e = cudaLaunchCooperativeKernel((const void*)kern, dim3(grid),
+                                      dim3(32 * FE_ITEM_WARPS * places), args, smem, s);
+    if (e != cudaSuccess) return cuda_status(e, "qsx_fe_heisenberg_rk4");
     QSX_LAUNCH_CHECK("qsx_fe_heisenberg_rk4");
     return QSX_OK;
   };
