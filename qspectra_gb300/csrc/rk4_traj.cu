@@ -6,8 +6,10 @@
 // With D_n = P^n - I the states come in doubling blocks instead,
 //   y_{n + j} = y_j + D_n y_j   (j < n),    D_{2n} = 2 D_n + D_n D_n,
 // log2 T dependent phases whose T m^2 + log2(T) m^3 multiply-adds are
-// independent within a phase and spread over every SM.  All of it runs in
-// FP64, for single-precision propagators too.
+// independent within a phase and spread over every SM.  Large blocks stop
+// squaring early and go on in blocks of that many states: a square of 252
+// elements costs as much as 250 states.  All of it runs in FP64, for
+// single-precision propagators too.
 //
 // The powers are kept transposed, DT[c][r] = D[r][c]: then a square and a
 // block of states are the same operation on rows x (of DT, or of states),
@@ -16,9 +18,10 @@
 //
 // Bound: FP64 issue (2 multiply-adds per clock and SM) once a phase fills the
 // chip, launch latency before that.  Whole calls in FP64, before and after: a
-// 7-site trajectory (49 elements, 1000 states) 8.52 and 0.53 ms, a 7-site
-// spectrum (7 elements, 2048 states) 5.11 and 1.27 ms, a dimer trajectory (4
-// elements, 120 states) 0.52 and 0.36 ms.
+// 7-site trajectory (49 elements, 1000 states) 8.52 and 0.45 ms, a 7-site
+// spectrum (7 elements, 2048 states) 5.11 and 1.24 ms, a dimer trajectory (4
+// elements, 120 states) 0.51 and 0.35 ms, a trimer hierarchy through its
+// dense propagator (252 elements, 500 states) 12.6 and 1.65 ms.
 //
 // A power can overflow, or meet a non-finite generator, where the stepped
 // loop would not (an unstable mode that the state does not excite).  Every
@@ -52,28 +55,52 @@ struct TrajJob {
   int rows, batch;
 };
 
-// sum_k DT[k][r] x[k] with two accumulators (the dependent multiply-adds of
-// one would leave the FP64 pipe idle in the small phases)
-__device__ __forceinline__ double2 traj_dot(const double2* dt, const double2* x, int m) {
-  double2 a0 = make_double2(0.0, 0.0), a1 = a0;
-  int k = 0;
-#pragma unroll 4
-  for (; k + 1 < m; k += 2) {
-    cfma(a0, dt[(int64_t)k * m], x[k]);
-    cfma(a1, dt[(int64_t)(k + 1) * m], x[k + 1]);
+// sum over k = k0, k0 + step, .. < m of DT[k][r] x[k], eight independent
+// chains of multiply-adds: a dependent one takes 140 clocks, an issue 16
+__device__ __forceinline__ double2 traj_dot(const double2* dt, const double2* x, int m, int k0 = 0,
+                                            int step = 1) {
+  double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  int k = k0;
+#pragma unroll 2
+  for (; k + step < m; k += 2 * step) {
+    const double2 d0 = dt[(int64_t)k * m], v0 = x[k];
+    const double2 d1 = dt[(int64_t)(k + step) * m], v1 = x[k + step];
+    a[0] = fma(d0.x, v0.x, a[0]);
+    a[1] = fma(-d0.y, v0.y, a[1]);
+    a[2] = fma(d0.x, v0.y, a[2]);
+    a[3] = fma(d0.y, v0.x, a[3]);
+    a[4] = fma(d1.x, v1.x, a[4]);
+    a[5] = fma(-d1.y, v1.y, a[5]);
+    a[6] = fma(d1.x, v1.y, a[6]);
+    a[7] = fma(d1.y, v1.x, a[7]);
   }
-  if (k < m) cfma(a0, dt[(int64_t)k * m], x[k]);
-  return cadd(a0, a1);
+  if (k < m) {
+    const double2 d0 = dt[(int64_t)k * m], v0 = x[k];
+    a[0] = fma(d0.x, v0.x, a[0]);
+    a[1] = fma(-d0.y, v0.y, a[1]);
+    a[2] = fma(d0.x, v0.y, a[2]);
+    a[3] = fma(d0.y, v0.x, a[3]);
+  }
+  return make_double2((a[0] + a[1]) + (a[4] + a[5]), (a[2] + a[3]) + (a[6] + a[7]));
 }
 
+// output e of the job by `parts` neighbouring lanes, this one's share k = part, ..
 template <bool SINGLE>
 __device__ __forceinline__ void traj_output(const TrajJob& job, const double2* dt_all,
-                                            int64_t dt_stride, int m, unsigned e, int* flag) {
+                                            int64_t dt_stride, int m, unsigned e, bool live,
+                                            int parts, int part, int* flag) {
   const unsigned r = e % m, row = e / m, j = row % job.rows, b = row / job.rows;
   const double2* x = job.x + b * job.x_stride + (int64_t)j * m;
+  double2 z = make_double2(0.0, 0.0);
+  if (live) z = traj_dot(dt_all + b * dt_stride + r, x, m, part, parts);
+  for (int o = 16; o >= 32 / parts; o >>= 1) {
+    z.x += __shfl_xor_sync(0xffffffffu, z.x, o);
+    z.y += __shfl_xor_sync(0xffffffffu, z.y, o);
+  }
+  if (!live || part) return;
   double2 v = x[r];
   if (job.add) v = cadd(v, job.add[b * job.add_stride + (int64_t)j * m + r]);
-  v = cadd(v, traj_dot(dt_all + b * dt_stride + r, x, m));
+  v = cadd(v, z);
   job.out[b * job.out_stride + (int64_t)j * m + r] = v;
   if (!state_finite<SINGLE>(v)) atomicOr(flag, 1);
 }
@@ -97,17 +124,26 @@ __global__ void __launch_bounds__(256)
   if (e == 0) *flag = 0;
 }
 
+// A warp takes 32 / parts consecutive outputs of one job: lane l the output
+// l % (32 / parts), its share l / (32 / parts) of the sum.
 template <bool SINGLE>
 __global__ void __launch_bounds__(TRAJ_THREADS)
     traj_phase_kernel(TrajJob rows, TrajJob power, const double2* DT, int64_t dt_stride, int m,
-                      int* flag) {
+                      int parts, int* flag) {
+  const unsigned per = 32 / parts, lane = threadIdx.x & 31;
   const unsigned nr = (unsigned)rows.rows * rows.batch * m;
   const unsigned np = (unsigned)power.rows * power.batch * m;
-  const unsigned e = blockIdx.x * TRAJ_THREADS + threadIdx.x;
-  if (e < nr)
-    traj_output<SINGLE>(rows, DT, dt_stride, m, e, flag);
-  else if (e < nr + np)
-    traj_output<false>(power, DT, power.x_stride, m, e - nr, flag);
+  const unsigned wr = (nr + per - 1) / per;   // warps of the first job
+  const unsigned w = blockIdx.x * (TRAJ_THREADS / 32) + threadIdx.x / 32;
+  const int part = lane / per;
+  if (w < wr) {
+    const unsigned e = w * per + lane % per;
+    traj_output<SINGLE>(rows, DT, dt_stride, m, min(e, nr - 1), e < nr, parts, part, flag);
+  } else {
+    const unsigned e = (w - wr) * per + lane % per;
+    if ((w - wr) * per >= np) return;   // whole warps
+    traj_output<false>(power, DT, power.x_stride, m, min(e, np - 1), e < np, parts, part, flag);
+  }
 }
 
 // Every phase in one launch, one CTA per sample, the powers in shared memory:
@@ -159,7 +195,7 @@ __global__ void __launch_bounds__(TRAJ_CTA_THREADS)
 // A + A^2/2 + A^3/6 + A^4/24 needs row r alone, r A (I + A/2 (I + A/3 (I + A/4)))
 // evaluated left to right, so m CTAs a sample share nothing.  Three products
 // where the two-product form of the batched kernel needs the whole of A^2 in
-// one CTA: 256 us for one 49 x 49 block, on one SM.
+// one CTA: 256 us for one 49 x 49 block, on one SM, where this takes 24.
 __global__ void __launch_bounds__(64)
     propagator_rows_kernel(const double2* __restrict__ L, int m, double h,
                            double2* __restrict__ D) {
@@ -199,7 +235,7 @@ int propagator_rows_run(const double2* L, int m, int64_t batch, double h, double
 int rk4_traj_plan(const qsx_rk4_args* a, TrajPlan* pl) {
   pl->form = TRAJ_NONE;
   const int64_t m = a->m, B = a->batch, nsave = a->nsteps / a->save_every + 1;
-  if (a->form != 0 || !a->out_state || a->nproj || a->nselect || a->block_k > 1 || m > 64 ||
+  if (a->form != 0 || !a->out_state || a->nproj || a->nselect || a->block_k > 1 || m > 512 ||
       a->variant || nsave < 8 || B < 1 || B * nsave * m >= (int64_t)1 << 31 ||
       (a->matrix_stride != 0 && B * m * m >= (int64_t)1 << 31))
     return QSX_OK;
@@ -224,15 +260,30 @@ int rk4_traj_plan(const qsx_rk4_args* a, TrajPlan* pl) {
           : a->nsteps * std::max(0.25, per_sm * 4.0 * m * m / (16.0 * sm_rate));
   // one launch, a CTA per sample
   const double waves = std::ceil(per_sm);
-  const double cta = a->save_every == 1
+  const double cta = a->save_every == 1 && m <= 64
                          ? 4.0 + waves * (0.6 * phases + (rows + phases * sq) / sm_rate)
                          : 1e30;
-  // a launch a phase, outputs spread over all SMs
-  const double spread = 4.0 + 3.0 * (phases + power) +
-                        (B * rows + mats * (phases + power) * sq) / (0.7 * sm_rate * sms);
+  // a launch a phase, outputs spread over all SMs: squares up to D_stop, then
+  // blocks of `stop` states
+  const double rate = 0.7 * sm_rate * sms;
+  double spread = 1e30;
+  double squares = 0.0;
+  const double phase = 3.0 + 0.01 * m;   // launch, and a shared sum's latency
+  for (int64_t stop = 1, q = 0; ; stop *= 2, ++q) {
+    const double blocks = (double)((nsave - stop + stop - 1) / stop);
+    const double t = 4.0 + (power + q + blocks) * phase + mats * power * sq / rate + squares +
+                     B * rows / rate;
+    if (t < spread) {
+      spread = t;
+      pl->stop = (int)stop;
+    }
+    if (stop >= nsave || stop >= (int64_t)1 << 30) break;
+    squares += mats * sq / rate;   // D_{2 stop}
+  }
   if (std::min(cta, spread) >= chain) return QSX_OK;
   pl->form = cta < spread ? TRAJ_CTA : TRAJ_SPREAD;
   pl->mats = mats;
+  pl->sms = sms;
   const int bufs = pl->form == TRAJ_CTA ? 0 : a->save_every > 1 ? 4 : 2;
   pl->bytes = 16 + (size_t)bufs * mats * m * m * sizeof(double2);
   return QSX_OK;
@@ -266,9 +317,16 @@ static int traj_run(const qsx_rk4_args* a, const TrajPlan& pl, cudaStream_t s) {
   QSX_LAUNCH_CHECK("qsx_rk4_batched trajectory init");
   const int64_t ms = pl.mats > 1 ? mm : 0;   // powers shared by all samples, or one each
   auto launch = [&](const TrajJob& rows, const TrajJob& power, const double2* dt) {
-    const int64_t n = ((int64_t)rows.rows * rows.batch + (int64_t)power.rows * power.batch) * m;
-    traj_phase_kernel<sizeof(C) == 8><<<(unsigned)((n + TRAJ_THREADS - 1) / TRAJ_THREADS), TRAJ_THREADS, 0, s>>>(
-        rows, power, dt, ms, m, flag);
+    // few outputs: lanes share each one's sum until every SM has four warps
+    // (or a share is down to eight terms)
+    const int64_t nr = (int64_t)rows.rows * rows.batch * m;
+    const int64_t np = (int64_t)power.rows * power.batch * m;
+    int parts = 1;
+    while (parts < 16 && (nr + np) * parts < (int64_t)pl.sms * 128 && m >= 16 * parts) parts *= 2;
+    const int64_t per = 32 / parts, warps = (nr + per - 1) / per + (np + per - 1) / per;
+    const int64_t wpc = TRAJ_THREADS / 32;
+    traj_phase_kernel<sizeof(C) == 8><<<(unsigned)((warps + wpc - 1) / wpc), TRAJ_THREADS, 0, s>>>(
+        rows, power, dt, ms, m, parts, flag);
   };
   const TrajJob none = {nullptr, nullptr, nullptr, 0, 0, 0, 0, 0};
   auto square = [&](const double2* dt, double2* out) {
@@ -297,12 +355,16 @@ static int traj_run(const qsx_rk4_args* a, const TrajPlan& pl, cudaStream_t s) {
     spare = cur;
     cur = res;
   }
-  for (int64_t n = 1; n < nsave; n *= 2) {
-    const int cnt = (int)std::min(n, nsave - n);
-    const TrajJob rows = {state, nullptr, state + n * m, nsave * m, 0, nsave * m,
-                          cnt, (int)a->batch};
-    launch(rows, 2 * n < nsave ? square(cur, spare) : none, cur);
-    std::swap(cur, spare);
+  for (int64_t n = 1; n < nsave;) {
+    // states n .. from the `block` before them
+    const int64_t block = std::min<int64_t>(n, pl.stop);
+    const int cnt = (int)std::min(block, nsave - n);
+    const TrajJob rows = {state + (n - block) * m, nullptr, state + n * m, nsave * m, 0,
+                          nsave * m, cnt, (int)a->batch};
+    const bool more = n < pl.stop && 2 * n < nsave;
+    launch(rows, more ? square(cur, spare) : none, cur);
+    if (more) std::swap(cur, spare);
+    n += cnt;
   }
   QSX_LAUNCH_CHECK("qsx_rk4_batched trajectory");
   return QSX_OK;

@@ -9,11 +9,13 @@ enum TrajForm { TRAJ_NONE = 0, TRAJ_CTA = 1, TRAJ_SPREAD = 2 };
 struct TrajPlan {
   TrajForm form;
   int64_t mats;   // distinct propagators
+  int stop;       // TRAJ_SPREAD: steps of the last power
+  int sms;
   size_t bytes;   // workspace: an int flag (16 bytes), then the powers
 };
 
 // The form for these arguments: TRAJ_NONE where the stepped loop is sooner
-// done, or where it is the only one (projections, stages, m > 64).
+// done, or where it is the only one (projections, stages, m > 512).
 int rk4_traj_plan(const qsx_rk4_args* a, TrajPlan* pl);
 // Runs it in a->workspace; the int at its start is nonzero afterwards (on the
 // device) when a value was not finite and the stepped loop has to run.
