@@ -20,6 +20,7 @@
 
 #include <algorithm>
 
+#include "heom_site.cuh"
 #include "qsx_common.cuh"
 #include "qsx_tc.cuh"
 
@@ -1721,7 +1722,16 @@ int qsx_heom_rk4(const qsx_heom_args* a, void* stream) {
       double2* saves = (double2*)(((size_t)ws + 255) & ~(size_t)255);
       double2* dst = node0 ? node0 : saves;
       int cst = QSX_OK;
-      if (heom_rk4_cluster<T>(a, dst, s, &cst)) {
+      // FP32 one-exciton blocks: the hierarchy on chip (heom_site.cu).  Its
+      // scratch: the low words where the other forms keep their states (past
+      // the saves), the order of the nodes at the end, in the site terms (64
+      // bytes a node at least)
+      const size_t save_bytes =
+          a->out_mean ? (size_t)p.batch * p.nsave * keep * p.E * sizeof(double2) : 0;
+      float2* low = (float2*)(((size_t)saves + save_bytes + 255) & ~(size_t)255);
+      int* order = (int*)((size_t)(ws + need - 8 * (size_t)p.nnodes) & ~(size_t)15);
+      if ((a->variant == 0 && sizeof(T) == 4 && heom_site_run(a, dst, low, order, s, &cst)) ||
+          heom_rk4_cluster<T>(a, dst, s, &cst)) {
         if (cst) return cst;
         if (a->out_mean) {
           const int64_t m = (int64_t)p.nsave * keep * p.E;
