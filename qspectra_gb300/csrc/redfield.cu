@@ -62,7 +62,9 @@ __device__ __forceinline__ void jacobi_rotation(float app, float aqq, float apq,
 // indices).  Symmetric update: a_pp -= t a_pq, a_qq += t a_pq, and for
 // k != p, q the pair (a_kp, a_kq) rotates by (c, s).
 // T = float runs the same sweeps in FP32 (for builds feeding FP32
-// propagation; stops at off-diagonal mass below 1e-13 of the diagonal).
+// propagation; stops at off-diagonal mass below 1e-13 of the diagonal).  The
+// matrix is scaled by a power of two so that no square leaves the range.
+// The block's rows of U are written whole, zero outside the block.
 template <typename T, int NB>
 __global__ void __launch_bounds__(64)
     eigh_block_kernel(const double* __restrict__ H, int n, int off, int64_t batch,
@@ -73,11 +75,17 @@ __global__ void __launch_bounds__(64)
   T A[NB][NB], V[NB][NB];
   const double* h = H + b * n * n;
   const T tol = sizeof(T) == 4 ? (T)1e-13 : (T)1e-32;
+  double top = 0.0;
+#pragma unroll
+  for (int i = 0; i < NB; ++i)
+#pragma unroll
+    for (int j = i; j < NB; ++j) top = fmax(top, fabs(h[(off + i) * n + off + j]));
+  const int ex = isfinite(top) && top > 0.0 ? ilogb(top) : 0;
 #pragma unroll
   for (int i = 0; i < NB; ++i)
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
-      if (j >= i) A[i][j] = (T)h[(off + i) * n + off + j];
+      if (j >= i) A[i][j] = (T)scalbn(h[(off + i) * n + off + j], -ex);
       V[i][j] = i == j ? (T)1 : (T)0;
     }
   for (int sweep = 0; sweep < 30; ++sweep) {
@@ -124,17 +132,311 @@ __global__ void __launch_bounds__(64)
 #pragma unroll
     for (int j = 0; j < NB; ++j)
       rank += (A[j][j] < A[i][i] || (A[j][j] == A[i][i] && j < i)) ? 1 : 0;
-    E[b * n + off + rank] = (double)A[i][i];
+    E[b * n + off + rank] = scalbn((double)A[i][i], ex);
 #pragma unroll
     for (int r = 0; r < NB; ++r) U[b * n * n + (off + r) * n + off + rank] = (double)V[r][i];
   }
+  for (int r = 0; r < NB; ++r)
+    for (int c = 0; c < n; ++c)
+      if (c < off || c >= off + NB) U[b * n * n + (off + r) * n + c] = 0.0;
 #undef AS
 }
 
-// zero the off-block entries of U (the block kernels write only their blocks)
-__global__ void zero_kernel(double* p, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = 0.0;
+// One warp per matrix, FP64 blocks of 2 to 8.  Bound: the latency of dependent
+// FP64 operations (about 70 ns each here).  One thread's FP64 sweeps are a
+// chain of 7 x 21 rotations of 35 such operations for 7 x 7.  Microseconds a
+// call for one or 300 matrices, thread form and this one: 28 / 23 for 3 x 3,
+// 137 / 34 for 5 x 5, 402 / 55 for 7 x 7, 577 / 63 for 8 x 8 (22 of them the
+// call).  So
+// * the sweeps run in FP32 first, in the same order (hence the same signs and
+//   the same places of the eigenvectors): the matrix in registers, the same in
+//   every lane, and a row of the eigenvectors a lane;
+// * X <- X (1 + R/2 + 3/8 R^2), R = 1 - X^T X, makes the basis orthonormal to
+//   FP64 rounding: R is 1e-6 and the step leaves R^3;
+// * S = X^T A X is off diagonal by 1e-7, and FP64 sweeps finish it, two of
+//   them unless levels nearly meet: all pairs of a round-robin round at once,
+//   the tangents to FP32 accuracy (an element shrinks by 1e-7 a rotation, the
+//   quadratic convergence does the same), cosines in FP64.
+// The matrix is scaled by a power of two into FP32's range.
+template <int NB>
+struct EighWarpSmem {
+  static constexpr int LD = NB + 1;
+  double S[NB * LD], X[NB * LD], T[NB * LD];
+};
+constexpr int EIGH_BLOCK_WARPS = 2;
+// Up to this many matrices the warp form is the faster one: a thread's chain
+// is about NB^3 long and hidden by the other matrices once they fill the chip,
+// where a warp per matrix spends more FP64 issue slots.  Measured, thread form
+// and warp form: 3 x 3, 10000 matrices 65 / 241 us; 7 x 7, 300: 403 / 57,
+// 10000: 498 / 560, 200000: 4588 / 9499; 8 x 8, 10000: 743 / 662.
+template <int NB>
+constexpr int64_t EIGH_WARP_MAX = 19 * NB * NB * NB;
+
+template <int NB>
+__global__ void __launch_bounds__(32 * EIGH_BLOCK_WARPS)
+    eigh_warp_kernel(const double* __restrict__ H, int n, int off, int64_t batch, double* E,
+                     double* U) {
+  constexpr int LD = NB + 1, NN = NB * NB;
+  constexpr int NP = (NB + 1) / 2 * 2, M = NP / 2;   // players (one idle when odd) and pairs
+  constexpr unsigned ALL = 0xffffffffu;
+  __shared__ EighWarpSmem<NB> smem[EIGH_BLOCK_WARPS];
+  const int lane = threadIdx.x & 31;
+  const int64_t b = (int64_t)blockIdx.x * EIGH_BLOCK_WARPS + threadIdx.x / 32;
+  if (b >= batch) return;
+  double *S = smem[threadIdx.x / 32].S, *X = smem[threadIdx.x / 32].X, *Y = smem[threadIdx.x / 32].T;
+  const double* h = H + b * n * n;
+  // ---- load the upper triangle, scale
+  double top = 0.0;
+  for (int e = lane; e < NN; e += 32) {
+    const int i = min(e / NB, e % NB), j = max(e / NB, e % NB);
+    const double a = h[(off + i) * n + off + j];
+    S[e / NB * LD + e % NB] = a;
+    top = isfinite(a) ? fmax(top, fabs(a)) : INFINITY;
+  }
+  for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(ALL, top, o));
+  const bool finite = isfinite(top);
+  const int ex = finite && top > 0.0 ? ilogb(top) : 0;
+  for (int e = lane; e < NN; e += 32) {
+    double& a = S[e / NB * LD + e % NB];
+    a = finite ? scalbn(a, -ex) : NAN;   // nothing can be said of such a matrix
+  }
+  __syncwarp();
+  // ---- FP32 sweeps
+  {
+#define AS(i, j) A[(i) < (j) ? (i) : (j)][(i) < (j) ? (j) : (i)]
+    float A[NB][NB], v[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+#pragma unroll
+      for (int j = i; j < NB; ++j) A[i][j] = (float)S[i * LD + j];
+      v[i] = i == lane ? 1.f : 0.f;
+    }
+    for (int sweep = 0; sweep < 12; ++sweep) {
+      float offd = 0.f, dia = 0.f;
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        dia = fmaf(A[i][i], A[i][i], dia);
+#pragma unroll
+        for (int j = i + 1; j < NB; ++j) offd = fmaf(A[i][j], A[i][j], offd);
+      }
+      if (!(offd > 1e-13f * dia)) break;
+#pragma unroll
+      for (int p = 0; p < NB - 1; ++p) {
+#pragma unroll
+        for (int q = p + 1; q < NB; ++q) {
+          const float apq = A[p][q];
+          if (apq != 0.f) {
+            float c, s, t;
+            jacobi_rotation(A[p][p], A[q][q], apq, c, s, t);
+            A[p][p] = fmaf(-t, apq, A[p][p]);
+            A[q][q] = fmaf(t, apq, A[q][q]);
+            A[p][q] = 0.f;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) {
+              if (k == p || k == q) continue;
+              const float g = AS(k, p), hh = AS(k, q);
+              AS(k, p) = c * g - s * hh;
+              AS(k, q) = s * g + c * hh;
+            }
+            const float vp = v[p], vq = v[q];
+            v[p] = c * vp - s * vq;
+            v[q] = s * vp + c * vq;
+          }
+        }
+      }
+    }
+#undef AS
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (lane < NB) X[lane * LD + j] = (double)v[j];
+  }
+  __syncwarp();
+  // ---- orthonormal to FP64: Y = R, then P = 1 + R/2 + 3/8 R^2, X <- X P
+  constexpr int PER = (NN + 31) / 32;
+  double w[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = lane + 32 * u, i = e / NB, j = e % NB;
+    double a0 = i == j ? 1.0 : 0.0, a1 = 0.0;
+    if (e < NN) {
+#pragma unroll
+      for (int k = 0; k < NB; ++k) {
+        double& a = k & 1 ? a1 : a0;
+        a = fma(-X[k * LD + i], X[k * LD + j], a);
+      }
+      Y[i * LD + j] = a0 + a1;
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = lane + 32 * u, i = e / NB, j = e % NB;
+    double a = 0.0;
+    if (e < NN) {
+#pragma unroll
+      for (int k = 0; k < NB; ++k) a = fma(Y[i * LD + k], Y[k * LD + j], a);
+      w[u] = fma(0.375, a, 0.5 * Y[i * LD + j]);
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = lane + 32 * u;
+    if (e < NN) Y[e / NB * LD + e % NB] = w[u];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = lane + 32 * u, i = e / NB, j = e % NB;
+    double a = 0.0;
+    if (e < NN) {
+#pragma unroll
+      for (int k = 0; k < NB; ++k) a = fma(X[i * LD + k], Y[k * LD + j], a);
+      w[u] = X[i * LD + j] + a;
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = lane + 32 * u;
+    if (e < NN) X[e / NB * LD + e % NB] = w[u];
+  }
+  __syncwarp();
+  // ---- S <- X^T S X
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = lane + 32 * u, i = e / NB, j = e % NB;
+    double a0 = 0.0, a1 = 0.0;
+    if (e < NN) {
+#pragma unroll
+      for (int k = 0; k < NB; ++k) {
+        double& a = k & 1 ? a1 : a0;
+        a = fma(S[i * LD + k], X[k * LD + j], a);
+      }
+      Y[i * LD + j] = a0 + a1;
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int e = lane + 32 * u, i = e / NB, j = e % NB;
+    double a0 = 0.0, a1 = 0.0;
+    if (e < NN && i <= j) {
+#pragma unroll
+      for (int k = 0; k < NB; ++k) {
+        double& a = k & 1 ? a1 : a0;
+        a = fma(X[k * LD + i], Y[k * LD + j], a);
+      }
+      S[i * LD + j] = S[j * LD + i] = a0 + a1;
+    }
+  }
+  __syncwarp();
+  // ---- FP64 sweeps
+  const int bi = lane / (2 * M), bj = lane / 2 % M, half = lane & 1;   // block of S, its column
+  const int vr = lane / M, vj = lane % M;                              // row of X, pair
+  for (int sweep = 0; sweep < 30; ++sweep) {
+    double offd = 0.0, dia = 0.0;
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int e = lane + 32 * u, i = e / NB, j = e % NB;
+      if (e < NN) {
+        const double a = S[i * LD + j];
+        if (i == j) dia = fma(a, a, dia);
+        else offd = fma(a, a, offd);
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      offd += __shfl_xor_sync(ALL, offd, o);
+      dia += __shfl_xor_sync(ALL, dia, o);
+    }
+    if (!(offd > 2e-32 * dia)) break;   // offd counts each pair twice
+    for (int round = 0; round < NP - 1; ++round) {
+      auto player = [&](int pair, int second) {
+        const int k = second ? round - pair + NP - 1 : round + pair;
+        return pair == 0 && second ? NP - 1 : k % (NP - 1);
+      };
+      // the rotation of pair lane % M
+      const int rp = player(lane % M, 0), rq = player(lane % M, 1);
+      double c = 1.0, s = 0.0, left = 0.0, up = 0.0;
+      if (rp < NB && rq < NB) {
+        const double apq = S[rp * LD + rq], d = S[rq * LD + rq] - S[rp * LD + rp];
+        if (apq != 0.0) {
+          const float tau = (float)d / (2.f * (float)apq);
+          const float tf = fabsf(tau) < 1e18f
+                               ? (tau >= 0.f ? 1.f : -1.f) / (fabsf(tau) + sqrtf(fmaf(tau, tau, 1.f)))
+                               : 0.5f / tau;
+          const float r0f = rsqrtf(fmaf(tf, tf, 1.f));
+          const double t = isfinite(tf) ? (double)tf : 0.0, r0 = isfinite(tf) ? (double)r0f : 1.0;
+          // c = (1 + t^2)^(-1/2): e = 1 - (1 + t^2) r0^2, c = r0 (1 + e/2 + 3/8 e^2)
+          const double rr = r0 * r0, e = fma(-rr, t * t, 1.0 - rr);
+          c = fma(r0 * e, fma(0.375, e, 0.5), r0);
+          s = t * c;
+          const double x = fma(t, d, -2.0 * apq);
+          left = c * c * (fma(-t, d, apq) - t * t * apq);   // what remains of a_pq
+          up = c * s * x;                                  // a_pp grows, a_qq shrinks by it
+        }
+      }
+      const double ci = __shfl_sync(ALL, c, bi < M ? bi : 0), si = __shfl_sync(ALL, s, bi < M ? bi : 0);
+      const double cj = __shfl_sync(ALL, c, bj), sj = __shfl_sync(ALL, s, bj);
+      const double lj = __shfl_sync(ALL, left, bj), uj = __shfl_sync(ALL, up, bj);
+      const double cv = __shfl_sync(ALL, c, vj), sv = __shfl_sync(ALL, s, vj);
+      const int pi = player(bi, 0), qi = player(bi, 1), pj = player(bj, 0), qj = player(bj, 1);
+      const int pv = player(vj, 0), qv = player(vj, 1);
+      double o0 = 0.0, o1 = 0.0;   // rows pi, qi of column pj (half 0) or qj of the block
+      if (bi < bj) {
+        const double b00 = pi < NB && pj < NB ? S[pi * LD + pj] : 0.0;
+        const double b01 = pi < NB && qj < NB ? S[pi * LD + qj] : 0.0;
+        const double b10 = qi < NB && pj < NB ? S[qi * LD + pj] : 0.0;
+        const double b11 = qi < NB && qj < NB ? S[qi * LD + qj] : 0.0;
+        const double x0 = half ? fma(sj, b00, cj * b01) : fma(cj, b00, -(sj * b01));
+        const double x1 = half ? fma(sj, b10, cj * b11) : fma(cj, b10, -(sj * b11));
+        o0 = fma(ci, x0, -(si * x1));
+        o1 = fma(si, x0, ci * x1);
+      } else if (bi == bj && pj < NB && qj < NB) {
+        o0 = half ? lj : S[pj * LD + pj] + uj;
+        o1 = half ? S[qj * LD + qj] - uj : lj;
+      }
+      double xp = 0.0, xq = 0.0;
+      if (vr < NB && pv < NB && qv < NB) {
+        xp = X[vr * LD + pv];
+        xq = X[vr * LD + qv];
+      }
+      __syncwarp();
+      const int col = half ? qj : pj;
+      if (bi < M && bi <= bj && col < NB && (bi < bj || (pj < NB && qj < NB))) {
+        if (pi < NB) S[pi * LD + col] = o0;
+        if (qi < NB) S[qi * LD + col] = o1;
+        if (bi < bj) {
+          if (pi < NB) S[col * LD + pi] = o0;
+          if (qi < NB) S[col * LD + qi] = o1;
+        }
+      }
+      if (vr < NB && pv < NB && qv < NB) {
+        X[vr * LD + pv] = fma(cv, xp, -(sv * xq));
+        X[vr * LD + qv] = fma(sv, xp, cv * xq);
+      }
+      __syncwarp();
+    }
+  }
+  // ---- ascending order inside the block (stable on ties), whole rows of U
+  const double ev = lane < NB ? S[lane * LD + lane] : 0.0;
+  int rank = 0;
+#pragma unroll
+  for (int j = 0; j < NB; ++j) {
+    const double o = S[j * LD + j];
+    rank += o < ev || (o == ev && j < lane) ? 1 : 0;
+  }
+  if (!finite) rank = lane;
+  if (lane < NB) E[b * n + off + rank] = scalbn(ev, ex);
+  double* u = U + b * n * n + (int64_t)off * n;
+#pragma unroll
+  for (int i = 0; i < NB; ++i) {
+    const int to = off + __shfl_sync(ALL, rank, i);
+    if (lane < NB) u[lane * n + to] = finite ? X[lane * LD + i] : NAN;
+  }
+  for (int c = lane; c < n; c += 32)
+    if (c < off || c >= off + NB)
+      for (int r = 0; r < NB; ++r) u[r * n + c] = 0.0;
 }
 
 __global__ void __launch_bounds__(32 * EIGH_WARPS)
@@ -1361,9 +1663,8 @@ int qsx_eigh_batched_prec(const double* H, int n, int64_t batch, int nblocks,
     QSX_LAUNCH_CHECK("qsx_eigh_batched");
     return QSX_OK;
   }
-  const int64_t total = batch * n * n;
-  zero_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(U, total);
   const unsigned grid = (unsigned)((batch + 63) / 64);
+  const unsigned wgrid = (unsigned)((batch + EIGH_BLOCK_WARPS - 1) / EIGH_BLOCK_WARPS);
   for (int k = 0; k < nblocks; ++k) {
     const int off = block_starts[k], nb = block_starts[k + 1] - off;
     switch (nb) {
@@ -1371,6 +1672,8 @@ int qsx_eigh_batched_prec(const double* H, int n, int64_t batch, int nblocks,
   case NB:                                                                           \
     if (precision == QSX_FP32)                                                       \
       eigh_block_kernel<float, NB><<<grid, 64, 0, st>>>(H, n, off, batch, E, U);     \
+    else if (NB >= 2 && batch <= EIGH_WARP_MAX<NB>)                                  \
+      eigh_warp_kernel<NB < 2 ? 2 : NB><<<wgrid, 32 * EIGH_BLOCK_WARPS, 0, st>>>(H, n, off, batch, E, U); \
     else                                                                             \
       eigh_block_kernel<double, NB><<<grid, 64, 0, st>>>(H, n, off, batch, E, U);    \
     break;
