@@ -22,9 +22,9 @@ __device__ __forceinline__ uint32_t op_offset(int r, int k, uint32_t sbo) {
   return (uint32_t)(r >> 3) * sbo + (uint32_t)(k >> 2) * LBO + (uint32_t)((r & 7) * 16 + (k & 3) * 4);
 }
 
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t sbo) {
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t sbo, uint32_t lbo = LBO) {
   uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)(LBO >> 4) << 16;
+  d |= (uint64_t)(lbo >> 4) << 16;
   d |= (uint64_t)(sbo >> 4) << 32;
   d |= 1ull << 46;  // descriptor version for tcgen05; no swizzle, base offset 0
   return d;
@@ -53,52 +53,6 @@ __device__ __forceinline__ void st_split4(unsigned char* hi, unsigned char* lo, 
   *reinterpret_cast<float4*>(lo + off) = l;
 }
 
-// Operand row `arow` (K-major) from this thread's CPT values at columns
-// c0..c0+CPT-1; columns at or above m must already be zero.
-template <int CPT>
-__device__ __forceinline__ void store_row(unsigned char* hi, unsigned char* lo, int arow, int c0,
-                                          int kp, uint32_t sbo, const float (&v)[CPT]) {
-#pragma unroll
-  for (int g = 0; g < CPT / 4; ++g)
-    if (c0 + 4 * g < kp)
-      st_split4(hi, lo, op_offset(arow, c0 + 4 * g, sbo), v[4 * g], v[4 * g + 1], v[4 * g + 2],
-                v[4 * g + 3]);
-}
-
-// Transposed operand: this thread holds row k = r of X (columns
-// c0..c0+CPT-1); B^T row n = column n of X.  Lanes 4q..4q+3 (rows r & ~3 ..
-// +3) transpose 4 x 4 blocks with two xor-shuffle rounds, then each lane
-// writes 16 bytes (four consecutive k) of one B^T row.  Odd quads take the
-// blocks in swapped pairs so that one store instruction covers all 32 banks.
-template <int CPT>
-__device__ __forceinline__ void store_cols(unsigned char* hi, unsigned char* lo, int r, int c0,
-                                           int np, int kp, uint32_t sbo, const float (&v)[CPT],
-                                           int lane) {
-  const bool odd = (lane >> 2) & 1, b1 = lane & 1, b2 = (lane >> 1) & 1;
-  const int kq = r & ~3;
-#pragma unroll
-  for (int jj = 0; jj < CPT / 4; ++jj) {
-    float a0 = odd ? v[4 * (jj ^ 1)] : v[4 * jj];
-    float a1 = odd ? v[4 * (jj ^ 1) + 1] : v[4 * jj + 1];
-    float a2 = odd ? v[4 * (jj ^ 1) + 2] : v[4 * jj + 2];
-    float a3 = odd ? v[4 * (jj ^ 1) + 3] : v[4 * jj + 3];
-    {
-      const float s0 = b2 ? a0 : a2, s1 = b2 ? a1 : a3;
-      const float q0 = __shfl_xor_sync(0xffffffffu, s0, 2);
-      const float q1 = __shfl_xor_sync(0xffffffffu, s1, 2);
-      if (b2) { a0 = q0; a1 = q1; } else { a2 = q0; a3 = q1; }
-    }
-    {
-      const float s0 = b1 ? a0 : a1, s1 = b1 ? a2 : a3;
-      const float q0 = __shfl_xor_sync(0xffffffffu, s0, 1);
-      const float q1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-      if (b1) { a0 = q0; a2 = q1; } else { a1 = q0; a3 = q1; }
-    }
-    const int n = c0 + 4 * (jj ^ (int)odd) + (lane & 3);
-    if (n < np && kq < kp) st_split4(hi, lo, op_offset(n, kq, sbo), a0, a1, a2, a3);
-  }
-}
-
 __device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t adesc, uint64_t bdesc,
                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -107,6 +61,17 @@ __device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t adesc, uint64_
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
       :
       : "r"(dtmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
+// the same product with A in tensor memory: row = lane, one TF32 value a column
+__device__ __forceinline__ void mma_tf32_ts(uint32_t dtmem, uint32_t atmem, uint64_t bdesc,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+      :
+      : "r"(dtmem), "r"(atmem), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
 // One 3xTF32 product chain into the accumulator, issued by one thread, then
@@ -125,6 +90,26 @@ __device__ __forceinline__ void issue_product(uint32_t dtmem, uint64_t a_hi, uin
     mma_tf32(dtmem, a_hi + step, b_hi + step, idesc, (s > 0 || accumulate) ? 1u : 0u);
     mma_tf32(dtmem, a_hi + step, b_lo + step, idesc, 1);
     mma_tf32(dtmem, a_lo + step, b_hi + step, idesc, 1);
+  }
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+               :
+               : "r"(mbar)
+               : "memory");
+}
+
+// the chain with A's two planes in tensor memory (columns a_hi, a_lo on)
+template <int KSTEPS>
+__device__ __forceinline__ void issue_product_ts(uint32_t dtmem, uint32_t a_hi, uint32_t a_lo,
+                                                 uint64_t b_hi, uint64_t b_lo, uint32_t idesc,
+                                                 uint32_t mbar, uint32_t lbo) {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+  for (int s = 0; s < KSTEPS; ++s) {
+    const uint64_t step = (uint64_t)(2 * lbo >> 4) * (uint64_t)s;
+    const uint32_t col = 8u * (uint32_t)s;
+    mma_tf32_ts(dtmem, a_hi + col, b_hi + step, idesc, s > 0 ? 1u : 0u);
+    mma_tf32_ts(dtmem, a_hi + col, b_lo + step, idesc, 1);
+    mma_tf32_ts(dtmem, a_lo + col, b_hi + step, idesc, 1);
   }
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                :
@@ -197,6 +182,60 @@ __device__ __forceinline__ void tmem_store(uint32_t taddr, const float (&v)[16])
         "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])),
         "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
       : "memory");
+}
+
+// N consecutive columns (a multiple of 8, at most 32) of this thread's lane
+template <int N>
+__device__ __forceinline__ void tmem_load_cols(uint32_t taddr, float (&v)[N]) {
+  static_assert(N % 8 == 0 && N >= 8 && N <= 32, "8, 16, 24 or 32 columns");
+  if constexpr (N == 32 || N == 16) {
+    tmem_load(taddr, v);
+  } else {
+    uint32_t r[24];
+    if constexpr (N == 24)
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+          "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%24];\n\t"
+          "tcgen05.ld.sync.aligned.32x32b.x8.b32 "
+          "{%16,%17,%18,%19,%20,%21,%22,%23}, [%25];\n\t"
+          "tcgen05.wait::ld.sync.aligned;"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+            "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+            "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+            "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23])
+          : "r"(taddr), "r"(taddr + 16)
+          : "memory");
+    else
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+          "tcgen05.wait::ld.sync.aligned;"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+            "=r"(r[7])
+          : "r"(taddr)
+          : "memory");
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
+  }
+}
+
+// N consecutive columns of this thread's lane (a multiple of 8); the caller
+// waits with tmem_store_wait
+template <int N>
+__device__ __forceinline__ void tmem_store_cols(uint32_t taddr, const float (&v)[N]) {
+#pragma unroll
+  for (int g = 0; g < N; g += 8)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 :
+                 : "r"(taddr + (uint32_t)g), "r"(__float_as_uint(v[g])),
+                   "r"(__float_as_uint(v[g + 1])), "r"(__float_as_uint(v[g + 2])),
+                   "r"(__float_as_uint(v[g + 3])), "r"(__float_as_uint(v[g + 4])),
+                   "r"(__float_as_uint(v[g + 5])), "r"(__float_as_uint(v[g + 6])),
+                   "r"(__float_as_uint(v[g + 7]))
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_store_wait() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 }  // namespace tc
