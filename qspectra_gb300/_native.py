@@ -238,7 +238,8 @@ def _check(status, what):
 
 
 def _stream():
-    return _c_vp(torch.cuda.current_stream().cuda_stream)
+    # the handle alone: building a Stream object costs microseconds a launch
+    return _c_vp(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _p(t):
@@ -258,9 +259,34 @@ def _need(t, dtype, name, ndim=None):
 
 
 def require_gpu():
-    if not torch.cuda.is_available():
+    if not (torch.cuda.is_initialized() or torch.cuda.is_available()):
         raise QsxError('qspectra_gb300 needs a CUDA GPU; none is visible')
     load()
+
+
+def upload(values, dtype=None, device='cuda'):
+    """A host array on the GPU without waiting for the work launched before
+    it: through pinned memory, which torch keeps until the copy is done (a
+    copy from pageable memory synchronises the stream)."""
+    t = torch.as_tensor(np.ascontiguousarray(values), dtype=dtype)
+    if torch.device(device).type == 'cpu':
+        return t
+    return t.pin_memory().to(device, non_blocking=True)
+
+
+def check_later(later):
+    """Read the status words that calls given ``later=`` left in it, with one
+    synchronisation, and raise what the first of them to fail would have."""
+    if later:
+        for value, (_, check) in zip(torch.cat([s for s, _ in later]).tolist(), later):
+            check(value)
+
+
+def _checked(status, check, later):
+    if later is None:
+        check(int(status.item()))
+    else:
+        later.append((status, check))
 
 
 # --------------------------------------------------------------- wrappers
@@ -818,15 +844,23 @@ def rk4_block_matrix(D, K, select):
     return out
 
 
+def _rk4_check(st):
+    if st & QSX_ERR_NONFINITE:
+        raise IntegratorError('non-finite state during RK4 integration')
+    if st & QSX_ERR_INVALID_ARG:
+        raise QsxError('qsx_rk4_batched: index table out of range')
+
+
 def rk4(matrix, y0, nsteps, save_every=1, form=0, h=0.0, precision=None,
         state=False, proj=None, select=None, per_sample=True, mean=False,
-        check_finite=True, workspace=None, block_k=0, variant=0):
+        check_finite=True, workspace=None, block_k=0, variant=0, later=None):
     """Batched RK4 time loop (see qsx_rk4_args in include/qsx.h).
 
     matrix: (B, m, m) complex64 (FP32) / complex128 (FP64), or (m, m) shared.
     y0: (B, m) or (m,) complex128.  proj: (P, m) or (B, P, m) complex128.
     select: sequence of state indices.  Returns a dict with 'state'
-    (B, nsave, m), 'proj' (B, nsave, P) and/or 'mean' (nsave, P).
+    (B, nsave, m), 'proj' (B, nsave, P) and/or 'mean' (nsave, P).  A list
+    ``later`` takes the check of the status word for check_later.
     """
     require_gpu()
     if precision is None:
@@ -903,11 +937,7 @@ def rk4(matrix, y0, nsteps, save_every=1, form=0, h=0.0, precision=None,
         a.workspace_bytes = workspace.numel()
     _check(lib.qsx_rk4_batched(ctypes.byref(a), _stream()), 'qsx_rk4_batched')
     if check_finite:
-        st = int(status.item())
-        if st & QSX_ERR_NONFINITE:
-            raise IntegratorError('non-finite state during RK4 integration')
-        if st & QSX_ERR_INVALID_ARG:
-            raise QsxError('qsx_rk4_batched: index table out of range')
+        _checked(status, _rk4_check, later)
     out['status'] = status
     return out
 
@@ -1075,8 +1105,15 @@ def fe_generator(M, H, pair_sites, unit_convert, precision=QSX_FP64):
     return Q
 
 
+def _fe_check(st):
+    if st & QSX_ERR_CUDA:
+        raise QsxError('fe propagation: a grid barrier timed out')
+    if st & QSX_ERR_NONFINITE:
+        raise IntegratorError('non-finite state in the fe propagation')
+
+
 def fe_heisenberg_rk4(Q, Ae, Me, pair_sites, y0, nsteps, h, precision=QSX_FP64,
-                      check_finite=True):
+                      check_finite=True, later=None):
     """States (B, nsteps+1, P*N) complex128 of the Heisenberg 'fe' RK4 loop."""
     require_gpu()
     cd = _cplx_dtype(precision)
@@ -1099,11 +1136,7 @@ def fe_heisenberg_rk4(Q, Ae, Me, pair_sites, y0, nsteps, h, precision=QSX_FP64,
                                      _p(out), _p(ws), ws.numel(), _p(status), _stream()),
            'qsx_fe_heisenberg_rk4')
     if check_finite:
-        st = int(status.item())
-        if st & QSX_ERR_CUDA:
-            raise QsxError('fe propagation: a grid barrier timed out')
-        if st & QSX_ERR_NONFINITE:
-            raise IntegratorError('non-finite state in the fe propagation')
+        _checked(status, _fe_check, later)
     return out
 
 
@@ -1113,19 +1146,18 @@ class CsrMap:
     def __init__(self, dense, device='cuda'):
         dense = np.asarray(dense, dtype=complex)
         self.shape = dense.shape
-        rows, cols = np.nonzero(dense)
-        order = np.lexsort((cols, rows))
-        rows, cols = rows[order], cols[order]
-        rowptr = np.zeros(dense.shape[0] + 1, dtype=np.int32)
-        np.add.at(rowptr, rows + 1, 1)
-        rowptr = np.cumsum(rowptr).astype(np.int32)
-        vals = dense[rows, cols]
-        if len(vals) == 0:  # keep valid pointers for an all-zero map
-            cols = np.zeros(1, dtype=np.int64)
-            vals = np.zeros(1, dtype=complex)
-        self.rowptr = torch.as_tensor(rowptr, device=device)
-        self.cols = torch.as_tensor(cols.astype(np.int32), device=device)
-        self.vals = torch.as_tensor(vals, dtype=torch.complex128, device=device)
+        rows, cols = np.nonzero(dense)     # by rows, then columns
+        rowptr = np.searchsorted(rows, np.arange(dense.shape[0] + 1))
+        n = max(len(rows), 1)              # keep valid pointers for an all-zero map
+        # values, columns and row starts in one upload
+        host = np.zeros(20 * n + 4 * len(rowptr), dtype=np.uint8)
+        host[:16 * len(rows)].view(complex)[:] = dense[rows, cols]
+        host[16 * n:16 * n + 4 * len(rows)].view(np.int32)[:] = cols
+        host[20 * n:].view(np.int32)[:] = rowptr
+        data = upload(host, device=device)
+        self.vals = data[:16 * n].view(torch.complex128)
+        self.cols = data[16 * n:20 * n].view(torch.int32)
+        self.rowptr = data[20 * n:].view(torch.int32)
 
     def __call__(self, x):
         """x (..., n_in) complex128 CUDA -> (..., n_out)."""
@@ -1249,7 +1281,12 @@ def rk4_step_adjoint(L, gD, h):
     return gL
 
 
-def eigh_large(H):
+def _eigh_check(st):
+    if st:
+        raise QsxError('qsx_eigh_large_batched: non-finite eigenvalue (non-finite input?)')
+
+
+def eigh_large(H, later=None):
     """Batched FP64 eigensolver (Householder + implicit QL) for any n <= 2048.
     H (B, n, n) float64 CUDA, symmetric.  Returns E ascending and U."""
     require_gpu()
@@ -1263,8 +1300,7 @@ def eigh_large(H):
     status = torch.zeros(1, dtype=torch.int32, device=H.device)
     _check(lib.qsx_eigh_large_batched(_p(H), n, B, _p(E), _p(U), _p(ws), ws.numel(),
                                       _p(status), _stream()), 'qsx_eigh_large_batched')
-    if int(status.item()):
-        raise QsxError('qsx_eigh_large_batched: non-finite eigenvalue (non-finite input?)')
+    _checked(status, _eigh_check, later)
     return E, U
 
 

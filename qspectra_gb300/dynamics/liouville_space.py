@@ -26,14 +26,14 @@ def liouville_subspace_index(liouville_subspace, full_subspace, n_sites,
         if letter in full_subspace:
             cuts[letter] = np.arange(size) + total
             total += size
-    keep = np.zeros((total, total), dtype=bool)
+    parts = []
     for block in liouville_subspace.split(','):
         row, col = block
         if row not in cuts or col not in cuts:
             raise SubspaceError("{}{} not in subspace '{}'".format(
                 row, col, full_subspace))
-        keep[np.ix_(cuts[row], cuts[col])] = True
-    return np.flatnonzero(keep.reshape(-1, order='F'))
+        parts.append((cuts[col][:, None] * total + cuts[row]).reshape(-1))
+    return parts[0] if len(parts) == 1 else np.unique(np.concatenate(parts))
 
 
 def all_liouville_subspaces(hilbert_subspace):
@@ -89,19 +89,34 @@ class LinearMap:
     """A fixed matrix applied along the last axis of a state, on the GPU.
 
     Stands in for the bound ``ndarray.dot`` methods that the reference's
-    operators expose; numpy inputs give numpy outputs.
+    operators expose; numpy inputs give numpy outputs.  One numpy vector and a
+    small matrix stay on the host: two uploads, a launch and a read cost 100
+    microseconds there, the product a few.
     """
+    HOST_MAX = 1 << 14       # matrix elements
 
     def __init__(self, matrix, scalar=False):
-        self.matrix = torch.as_tensor(np.asarray(matrix, dtype=complex),
-                                      device=_device())
+        _native.require_gpu()
+        self._host = np.array(matrix, dtype=complex)
+        self._matrix = None
         self.scalar = scalar  # one output row returned as a scalar (expectation)
 
     @property
+    def matrix(self):
+        """The matrix on the GPU."""
+        if self._matrix is None:
+            self._matrix = torch.as_tensor(self._host, device=_device())
+        return self._matrix
+
+    @property
     def shape(self):
-        return tuple(self.matrix.shape)
+        return self._host.shape
 
     def __call__(self, state):
+        if (not isinstance(state, torch.Tensor) and np.ndim(state) == 1
+                and self._host.size <= self.HOST_MAX):
+            y = self._host @ np.asarray(state, dtype=complex)
+            return y[..., 0] if self.scalar else y
         x, is_tensor = _as_device(state)
         y = x @ self.matrix.T
         if self.scalar:

@@ -16,7 +16,7 @@ from .constants import GAUSSIAN_SD_FWHM
 from .operator_tools import (SubspaceError, basis_transform_operator,
                              basis_transform_vector, hilbert_subspace_index,
                              occupation_table, operator_extend,
-                             transition_operator, unit_vec)
+                             transition_sum, unit_vec)
 from .polarization import polarization_vector
 
 
@@ -157,9 +157,7 @@ class ElectronicHamiltonian:
         if self.dipoles is None:
             raise HamiltonianError('transition dipole moments undefined')
         proj = self.dipoles @ polarization_vector(polarization)
-        return sum(proj[n] * transition_operator(n, self.n_sites, subspace,
-                                                 transitions)
-                   for n in range(self.n_sites))
+        return transition_sum(proj, self.n_sites, subspace, transitions)
 
     # ---- eigen-structure (host set-up) -----------------------------------
     def eig(self, subspace):

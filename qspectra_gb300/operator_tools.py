@@ -101,6 +101,40 @@ def transition_operator(n, n_sites, subspace='gef', include_transitions='-+'):
     return out
 
 
+def pair_sites(n_sites):
+    """Sites (i, j), i < j, of the pair states in the order of all_states."""
+    count = np.arange(n_sites - 1, -1, -1)
+    i = np.repeat(np.arange(n_sites), count)
+    j = np.arange(len(i)) - np.repeat(np.cumsum(count) - count, count) + i + 1
+    return i, j
+
+
+def transition_sum(weights, n_sites, subspace='gef', include_transitions='-+'):
+    """Sum over the sites n of weights[n] times transition_operator(n, ...)."""
+    weights = np.asarray(weights)
+    sizes = n_excitations(n_sites)
+    start, total = {}, 0
+    for letter, size in zip(MANIFOLDS, sizes):
+        if letter in subspace:
+            start[letter] = total
+            total += int(size)
+    out = np.zeros((total, total), dtype=np.result_type(weights.dtype, float))
+    sites = np.arange(n_sites)
+    up = []                                   # (upper state, lower state, site)
+    if 'g' in start and 'e' in start:
+        up.append((start['e'] + sites, start['g'], sites))
+    if 'e' in start and 'f' in start:
+        i, j = pair_sites(n_sites)
+        pair = start['f'] + np.arange(len(i))
+        up += [(pair, start['e'] + i, j), (pair, start['e'] + j, i)]
+    for hi, lo, n in up:
+        if '+' in include_transitions:
+            out[hi, lo] = weights[n]
+        if '-' in include_transitions:
+            out[lo, hi] = weights[n]
+    return out
+
+
 def occupation_table(n_sites, subspace='gef'):
     """occ[i, s] = 1 when site i is excited in state s.
 

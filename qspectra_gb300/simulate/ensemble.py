@@ -14,7 +14,7 @@ from .. import _native
 from ..constants import GAUSSIAN_SD_FWHM
 from ..dynamics.redfield import RedfieldModel
 from ..hamiltonian import ElectronicHamiltonian
-from ..operator_tools import hilbert_subspace_index
+from ..operator_tools import hilbert_subspace_index, pair_sites
 
 
 def disorder_offsets(ham, size, start=0):
@@ -62,20 +62,18 @@ class SampleBatch:
 
     def H(self, subspace):
         ham = self.model.hamiltonian
-        base = torch.as_tensor(ham.H(subspace), dtype=torch.float64).cuda()
+        base = _native.upload(ham.H(subspace), torch.float64)
         n = base.shape[0]
-        H = base.expand(self.size, n, n).clone()
         if 'e' in subspace:
             sl = hilbert_subspace_index('e', subspace, ham.n_sites)
-            idx = torch.arange(sl.start, sl.stop, device=H.device)
-            H[:, idx, idx] += self.offsets
+            H = _native.disordered_hamiltonians(
+                base, self.offsets.expand(self.size, ham.n_sites).contiguous(), sl.start)
+        else:
+            H = base.expand(self.size, n, n).clone()
         if 'f' in subspace:
             sl = hilbert_subspace_index('f', subspace, ham.n_sites)
-            pairs = [(i, j) for i in range(ham.n_sites) for j in range(i + 1, ham.n_sites)]
-            ii = torch.as_tensor([p[0] for p in pairs], device=H.device)
-            jj = torch.as_tensor([p[1] for p in pairs], device=H.device)
-            idx = torch.arange(sl.start, sl.stop, device=H.device)
-            H[:, idx, idx] += self.offsets[:, ii] + self.offsets[:, jj]
+            ii, jj = _native.upload(np.array(pair_sites(ham.n_sites)))
+            H.diagonal(dim1=1, dim2=2)[:, sl] += self.offsets[:, ii] + self.offsets[:, jj]
         return H.contiguous()
 
 
@@ -512,9 +510,8 @@ def ensemble_linear_signal(model, time_max, ensemble_size, polarization='xx',
         if q is None:
             V0 = model.dipole_operator(sp0, polarization[0], '+')
             V1 = model.dipole_operator(sp1, polarization[1], '-')
-            y0 = torch.as_tensor(-V1.bra_vector, dtype=torch.complex128).cuda()
-            proj = torch.as_tensor(np.asarray(V0.commutator(rho0))[None, :],
-                                   dtype=torch.complex128).cuda()
+            y0 = _native.upload(-V1.bra_vector, torch.complex128)
+            proj = _native.upload(np.asarray(V0.commutator(rho0))[None, :], torch.complex128)
         else:
             axes = np.eye(3)
             P0 = np.array([model.dipole_operator(sp0, a, '+').commutator(rho0) for a in axes])
@@ -558,7 +555,7 @@ def ensemble_populations(model, initial_state, duration, ensemble_size,
     else:
         nn = int(round(np.sqrt(M)))
         select = [i * nn + i for i in range(nn)]
-    y0t = torch.as_tensor(y0, dtype=torch.complex128).cuda()
+    y0t = _native.upload(y0, torch.complex128)
     n_total = model.hamiltonian.n_states(model.hilbert_subspace)
     nb = can_use_hermitian(prec, idx, n_total, y0, len(t) - 1, build.site_ops)
     if nb is not None:

@@ -212,8 +212,7 @@ class ThirdOrderEngine:
         """Bra vector of the dipole operator: (n,) shared or (S, n) per sample."""
         if isinstance(vec, tuple):
             v = self._op(spec, vec, tr).bra_vector
-            return torch.as_tensor(np.asarray(v, dtype=complex),
-                                   dtype=torch.complex128).cuda()
+            return _native.upload(np.asarray(v, dtype=complex))
         basis = torch.as_tensor(np.array(
             [np.asarray(self._op(spec, tuple(np.eye(3)[a]), tr).bra_vector, dtype=complex)
              for a in range(3)]), dtype=torch.complex128).cuda()
@@ -229,15 +228,15 @@ class ThirdOrderEngine:
         return (vec.to(basis.dtype)[:, :, None] * basis[None]).sum(1).contiguous()
 
     # -------------------------------------------------------------- builds
-    def _f_operators(self, batch, build_e, cdt):
+    def _f_operators(self, batch, build_e, cdt, later=None):
         """Q (S, P, N, P) column operators of the 'fe' block in precision."""
         model, N, P = self.model, self.N, self.P
         ham = model.hamiltonian
         pair_sites, site_pairs = pair_tables(N)
-        self._pair_sites = torch.as_tensor(pair_sites).cuda()
-        sp = torch.as_tensor(site_pairs).cuda()
+        self._pair_sites = _native.upload(pair_sites)
+        sp = _native.upload(site_pairs)
         Hf = batch.H('f')
-        Ef, Uf = _native.eigh_large(Hf)
+        Ef, Uf = _native.eigh_large(Hf, later)
         Y = _native.fblock_tensor(Ef, Uf, N, sp, ham.bath, model.unit_convert, self.prec,
                                   model.discard_imag_corr,
                                   ham.bath.matsubara_cutoff)
@@ -281,10 +280,11 @@ class ThirdOrderEngine:
         build = RedfieldBuild(Hge, N, 'ge', occupation_table(N, 'ge'), ham.bath, uc,
                               False, model.discard_imag_corr, 'site')
         need_fe = 'ESA' in self.signals
+        later = []      # status words, read together once everything is launched
         if need_fe:
             Me = build.M[:, :, 1:, 1:].to(cdt).contiguous()
             Ae = (build.G[:, 1:, 1:] + 1j * uc * Hge[:, 1:, 1:]).to(cdt).contiguous()
-            Q = self._f_operators(batch, build, cdt)
+            Q = self._f_operators(batch, build, cdt, later)
         _tick(events, 't3')
         # ---- t3 legs (Heisenberg picture), shared by the geometries
         T3 = len(self.t3)
@@ -293,11 +293,12 @@ class ThirdOrderEngine:
         for d in ch3:
             y_eg = self._bra('eg->gg', ch[3][d], '-', S)
             v_eg[d] = _native.rk4(D3, y_eg, T3 - 1, 1, h=dt, precision=prec,
-                                  state=True)['state']                    # (S, T3, N)
+                                  state=True, later=later)['state']                    # (S, T3, N)
             if need_fe:
                 y_fe = self._bra('fe->ee', ch[3][d], '-', S)
                 v_fe[d] = _native.fe_heisenberg_rk4(Q, Ae, Me, self._pair_sites, y_fe,
-                                                    T3 - 1, dt, prec)     # (S, T3, P N)
+                                                    T3 - 1, dt, prec,
+                                                    later=later)          # (S, T3, P N)
         if need_fe:
             del Q
         W, g3 = {}, {}
@@ -358,7 +359,7 @@ class ThirdOrderEngine:
             for a in ch0:
                 v0 = self._ket0('gg->' + sub1, ch[0][a], geo[0])          # (N,) / (S, N)
                 rho1[a] = _native.rk4(D1, v0, T1 - 1, 1, h=dt, precision=prec,
-                                      state=True)['state']                 # (S, T1, N)
+                                      state=True, later=later)['state']    # (S, T1, N)
             total = torch.zeros((T1, len(gaps), T3), dtype=torch.complex128, device='cuda')
             if Wt is not None:
                 r = torch.stack([self._apply(sub1 + '->ee', geo[1], ch[1][b], rho1[a])
@@ -385,6 +386,7 @@ class ThirdOrderEngine:
                                                        g.contiguous())[0]
             out[geo] = total
         _tick(events, 'end')
+        _native.check_later(later)
         return out
 
 

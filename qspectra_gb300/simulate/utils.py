@@ -343,10 +343,14 @@ def fft_frequencies(t, rw_freq=0, unit_convert=1, sign=1, convention='angular'):
         unit_convert = unit_convert / (2 * np.pi)
     elif convention != 'linear':
         raise ValueError("convention must be 'angular' or 'linear'")
-    t_sym, _ = symmetric_grid(t)
+    return _grid_frequencies(symmetric_grid(t)[0], rw_freq, unit_convert, sign)
+
+
+def _grid_frequencies(t_sym, rw_freq, cycles, sign):
+    """FFT frequencies of a symmetric grid in units of 1 / ``cycles``."""
     n = t_sym.size
     dt = t_sym[1] - t_sym[0]
-    f = np.fft.fftshift(np.fft.fftfreq(n, dt * unit_convert))
+    f = np.fft.fftshift(np.fft.fftfreq(n, dt * cycles))
     if sign == 1:
         f = -f[::-1]
     return f + rw_freq
@@ -374,7 +378,8 @@ def fourier_transform(t, x, axis=-1, rw_freq=0, unit_convert=1, sign=1,
     origin = t_sym[t_sym.size // 2]  # sample ifftshift moves to index 0
     uc = unit_convert if convention == 'angular' else 2 * np.pi * unit_convert
     if freqs is None:
-        f = fft_frequencies(t, rw_freq, unit_convert, sign, convention)
+        cycles = unit_convert / (2 * np.pi) if convention == 'angular' else unit_convert
+        f = _grid_frequencies(t_sym, rw_freq, cycles, sign)
     else:
         f = np.asarray(freqs, float)
     as_numpy = not isinstance(x, torch.Tensor)
