@@ -130,12 +130,13 @@ __global__ void fe_generator_kernel(const T* __restrict__ M, const double* __res
 struct FeP {
   int P, N;
   const void* Q;          // [batch][P][N][P] complex (T)
-  const void* R;          // [batch][N b][N site][N c] complex (T), see fe_rows_kernel
+  const void* R;          // [batch][N b][N c][N site] complex (T), see fe_rows_kernel
   const int* pair_sites;  // [P][2]
   double h;
 };
 
-// The row operators by column: R[b][site][c] = conj(Me[site][c][b] - Ae[c][b] / 2)
+// The row operators by column: R[b][c][site] = conj(Me[site][c][b] - Ae[c][b] / 2);
+// lanes on consecutive pairs read consecutive sites
 template <typename T>
 __global__ void fe_rows_kernel(const typename cplx<T>::type* __restrict__ Me,
                                const typename cplx<T>::type* __restrict__ Ae, int N, int64_t batch,
@@ -143,7 +144,7 @@ __global__ void fe_rows_kernel(const typename cplx<T>::type* __restrict__ Me,
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nn = (int64_t)N * N;
   if (e >= batch * nn * N) return;
   const int64_t s = e / (nn * N);
-  const int b = (int)(e / nn % N), site = (int)(e / N % N), c = (int)(e % N);
+  const int b = (int)(e / nn % N), c = (int)(e / N % N), site = (int)(e % N);
   const typename cplx<T>::type m = Me[(s * N + site) * nn + (int64_t)c * N + b];
   const typename cplx<T>::type a = Ae[s * nn + (int64_t)c * N + b];
   R[e] = cmk(m.x - (T)0.5 * a.x, -(m.y - (T)0.5 * a.y));
@@ -167,7 +168,7 @@ __device__ __forceinline__ void fe_mac(double2 (&k)[1], double2 q, double2 x) { 
 // time: Q is read once a stage, so the bound is its traffic, and a group is as
 // many samples as leave Q in the L2 through all their stages (7 of 24 sites,
 // 102 MB).  A launch a stage over all 32 samples streamed Q from HBM at 5.0
-// TB/s, 93 us; 72 us in groups.  (One CTA a column, a launch a stage, 113 us.
+// TB/s, 93 us; 66 us in groups.  (One CTA a column, a launch a stage, 113 us.
 // Two or four independent teams of half- or quarter-size CTAs, one's barrier
 // behind the other's loads: 78 and 100 us, their items too few to come out
 // even.)
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(FE_THREADS, 1) fe_loop_kernel(FeP p, FeLoop l)
             for (int v = 0; v < V; ++v) {
               const int kk = p.pair_sites[2 * (row + v)], ll = p.pair_sites[2 * (row + v) + 1];
               for (int c = w; c < N; c += FE_ITEM_WARPS) {
-                const C ra = sR[kk * N + c], rb = sR[ll * N + c];
+                const C ra = sR[c * N + kk], rb = sR[c * N + ll];
                 cfma(k[v], __ldcg(x + (int64_t)c * P + row + v), cmk(ra.x + rb.x, ra.y + rb.y));
               }
             }
@@ -351,6 +352,285 @@ __global__ void __launch_bounds__(FE_THREADS, 1) fe_loop_kernel(FeP p, FeLoop l)
   if (!ok && l.status) atomicOr(l.status, QSX_ERR_NONFINITE);
 }
 
+// The loop with Q on chip.  Every stage reads all of Q, so past the sizes of
+// one CTA its traffic bounds the loop wherever Q lies: from the L2 6.6 TB/s.
+// Here a team of CTAs, one an SM, holds a sample's Q in shared memory and
+// registers through all its steps, and the teams work through the samples.
+//
+// A CTA owns consecutive elements of X (column by column, `rows` of them) and
+// for each the P values Q[.][b][row], laid out one element a row; warp w holds
+// `rs` of its rows in shared memory and RREG in registers.  The lanes split the
+// sum over q, each with its part of X's column in registers, and four rows at a
+// time add up through shuffles.  The row term, a sum over the columns of X, is
+// split over all warps, from the L2, its operators T_k + T_l in shared memory.
+// Thread i then holds the state, its low word and the stage sum of element i.
+// X crosses between the CTAs of a team once a stage, through the L2 and a
+// barrier of the team.
+//
+// Bound: latency.  Of a stage of 5.7 us (three teams of 50 CTAs, 24 sites) the
+// round trip of X takes 2.0, the column terms 2.5 and the row terms 1.2; 16
+// warps of 128 registers took 7.1, their row terms with operators from the L1.
+// us a stage, the loop over the L2 against this one: 24 sites, FP32, 1 / 3 / 32
+// samples 10.2 / 12.2 / 66 and 4.1 / 6.1 / 61; 20 sites 7.2 / 9.9 / 85 and 3.5 /
+// 4.6 / 31; 13 sites, 32 samples 15.5 and 6.2; FP64, one sample of 16 / 20 / 22
+// sites 13 / 32 / 46 and 6.7 / 9.9 / 16.
+constexpr int FE_TEAM_WARPS = 8, FE_TEAM_THREADS = 32 * FE_TEAM_WARPS;
+constexpr int FE_TEAM_CT = 8;     // columns of a row-term task
+constexpr int FE_TEAM_RREG = 6;   // FP32 rows that a warp can keep in registers
+
+struct FeTeam {
+  int64_t batch, y0_stride;
+  int csize, teams;      // CTAs of a team, teams
+  int rows, rw, rs;      // elements a CTA, rows a warp, of them in shared memory
+  int nb, parts, nsteps; // columns that a CTA's elements touch, parts of a row term
+  const double2* y0;
+  void* x;               // [teams][2][P N] complex (T): stage inputs
+  double2* out;
+  int* status;
+  unsigned* barrier;     // [teams][2] zeroed: arrivals, abort word
+};
+
+template <typename T, int NQ, int RREG>
+__global__ void __launch_bounds__(FE_TEAM_THREADS, 1) fe_team_kernel(FeP p, FeTeam t) {
+  using C = typename cplx<T>::type;
+  constexpr bool SPLIT = sizeof(T) == 4;
+  constexpr unsigned ALL = 0xffffffffu;
+  constexpr int CT = FE_TEAM_CT;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int P = p.P, N = p.N, per = P * N, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  C* sQ = (C*)smraw;                                  // [warps][rs][P]
+  C* sx = sQ + (size_t)FE_TEAM_WARPS * t.rs * P;      // [nb P] the columns of the input
+  C* kq = sx + (size_t)t.nb * P;                      // [rows] column terms
+  C* part = kq + t.rows;                              // [parts][rows] row terms
+  const int team = blockIdx.x / t.csize;
+  const int rho0 = blockIdx.x % t.csize * t.rows, nr = max(0, min(t.rows, per - rho0));
+  const int b0 = min(rho0, per - 1) / P, nx = min(t.nb * P, per - b0 * P);
+  // this warp's rows; the column of the first one and where the next begins
+  const int first = w * t.rw, bf = min(rho0 + first, per - 1) / P;
+  const C* wQ = sQ + (size_t)w * t.rs * P;
+  C* sW = part + t.parts * t.rows;                    // [N][rows] row operators T_k + T_l
+  // row terms: 32 elements of X and CT columns a task
+  const int chunks = max(1, (nr + 31) / 32), tasks = nr ? chunks * t.parts : 0;
+  const bool own = tid < nr;
+  const int me = rho0 + tid;
+  C* xbuf = (C*)t.x + (size_t)team * 2 * per;
+  const T h = (T)p.h, s6 = h / (T)6;
+  unsigned target = 0;
+  bool ok = true;
+  for (int64_t s = team; s < t.batch; s += t.teams) {
+    const C* Qg = (const C*)p.Q + s * (int64_t)per * P + rho0;
+    const C* Rg = (const C*)p.R + s * (int64_t)N * N * N;
+    double2* o = t.out + s * (t.nsteps + 1) * (int64_t)per;
+    const int held = FE_TEAM_WARPS * t.rs;
+    for (int e = tid; e < held * P; e += FE_TEAM_THREADS) {
+      const int i = e % held, q = e / held, local = i / t.rs * t.rw + i % t.rs;
+      sQ[(size_t)i * P + q] = local < nr ? Qg[(int64_t)q * per + local] : cmk((T)0, (T)0);
+    }
+    C qr[RREG ? RREG : 1][NQ];
+#pragma unroll
+    for (int i = 0; i < RREG; ++i)
+#pragma unroll
+      for (int j = 0; j < NQ; ++j) {
+        const int q = lane + 32 * j, local = first + t.rs + i;
+        qr[i][j] = (i + t.rs < t.rw && local < nr && q < P) ? Qg[(int64_t)q * per + local]
+                                                            : cmk((T)0, (T)0);
+      }
+    for (int e = tid; e < N * nr; e += FE_TEAM_THREADS) {
+      const int c = e / nr, rl = e % nr, row = (rho0 + rl) % P;
+      const C* r = Rg + ((size_t)((rho0 + rl) / P) * N + c) * N;
+      sW[c * t.rows + rl] = cadd2(r[p.pair_sites[2 * row]], r[p.pair_sites[2 * row + 1]]);
+    }
+    C yh = cmk((T)0, (T)0), yl = yh, ac = yh;
+    if (own) {
+      const double2 v = t.y0[s * t.y0_stride + me];
+      yh = cmk((T)v.x, (T)v.y);
+      if (SPLIT) yl = cmk((T)(v.x - (double)yh.x), (T)(v.y - (double)yh.y));
+      xbuf[me] = yh;
+      o[me] = v;
+    }
+    target += t.csize;
+    if (!fe_grid_barrier(t.barrier + 2 * team, target, t.status)) return;
+    int cur = 0;
+    for (int step = 1; step <= t.nsteps; ++step) {
+#pragma unroll 1
+      for (int stage = 0; stage < 4; ++stage, cur ^= 1) {
+        const C* in = xbuf + (size_t)cur * per;
+        for (int e = tid; e < nx; e += FE_TEAM_THREADS) sx[e] = __ldcg(in + b0 * P + e);
+        __syncthreads();
+        // odd warps form row terms before their column terms, even warps after:
+        // the trips to the L2 lie under the others' sums
+        auto row_terms = [&] {
+          for (int i = w; i < tasks; i += FE_TEAM_WARPS) {
+            const int pt = i / chunks, rl = i % chunks * 32 + lane;
+            if (rl >= nr) continue;
+            const C* at = in + (size_t)pt * CT * P + (rho0 + rl) % P;
+            const C* u = sW + (size_t)pt * CT * t.rows + rl;
+            C x[CT], k = cmk((T)0, (T)0);
+            const int n = N - pt * CT;
+#pragma unroll
+            for (int c = 0; c < CT; ++c) x[c] = c < n ? __ldcg(at + (size_t)c * P) : cmk((T)0, (T)0);
+#pragma unroll
+            for (int c = 0; c < CT; ++c) cfma(k, x[c], u[min(c, n - 1) * t.rows]);
+            part[pt * t.rows + rl] = k;
+          }
+        };
+        if (w & 1) row_terms();
+        if (first < nr) {
+          C xr[NQ];
+          int b = bf, bend = (bf + 1) * P - rho0;
+          auto column = [&] {
+#pragma unroll
+            for (int j = 0; j < NQ; ++j) {
+              const int q = lane + 32 * j;
+              xr[j] = q < P ? sx[(b - b0) * P + q] : cmk((T)0, (T)0);
+            }
+          };
+          column();
+          // the sums of R rows over the lanes: halves of the 2 R words change
+          // sides until each lane holds a part of one word
+          auto add_up = [&](auto& k, int local, int count) {
+            constexpr int R = sizeof(k) / sizeof(C);
+            T v[2 * R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+              v[2 * i] = k[i].x;
+              v[2 * i + 1] = k[i].y;
+            }
+            constexpr int STEP = 32 / (2 * R);     // lanes that share a word
+#pragma unroll
+            for (int n = R; n >= 1; n /= 2) {
+              const bool hi = lane & (STEP * n);
+#pragma unroll
+              for (int i = 0; i < n; ++i) {
+                const T keep = hi ? v[i + n] : v[i], give = hi ? v[i] : v[i + n];
+                v[i] = keep + __shfl_xor_sync(ALL, give, STEP * n);
+              }
+            }
+#pragma unroll
+            for (int n = STEP / 2; n >= 1; n /= 2) v[0] += __shfl_xor_sync(ALL, v[0], n);
+            const int at = lane / STEP;
+            if (lane % STEP == 0 && at / 2 < count && local + at / 2 < nr)
+              reinterpret_cast<T*>(kq)[2 * local + at] = v[0];
+          };
+          constexpr int R = 4;
+#pragma unroll 1
+          for (int i0 = 0; i0 < t.rs; i0 += R) {
+            C k[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) k[i] = cmk((T)0, (T)0);
+            const C* q = wQ + (size_t)i0 * P + lane;
+            const int last = min(R, t.rs - i0) - 1;
+            if (first + i0 + last < min(nr, bend) && (SPLIT || last == R - 1)) {
+              // past P: what follows, times 0; past the last row: that row again
+              const C* qi[R];
+#pragma unroll
+              for (int i = 0; i < R; ++i) qi[i] = q + min(i, last) * P;
+#pragma unroll
+              for (int j = 0; j < NQ; ++j)
+#pragma unroll
+                for (int i = 0; i < R; ++i) cfma(k[i], qi[i][32 * j], xr[j]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < R; ++i) {
+                if (i0 + i >= t.rs || first + i0 + i >= nr) continue;
+                if (first + i0 + i >= bend) {
+                  ++b;
+                  bend += P;
+                  column();
+                }
+#pragma unroll
+                for (int j = 0; j < NQ; ++j) cfma(k[i], q[i * P + 32 * j], xr[j]);
+              }
+            }
+            add_up(k, first + i0, t.rs - i0);   // rows past rs are others'
+          }
+          if constexpr (RREG > 0) {
+            constexpr int R2 = RREG > 4 ? 8 : 4;
+            static_assert(RREG <= 8, "one batch of register rows");
+            C k[R2];
+#pragma unroll
+            for (int i = 0; i < R2; ++i) k[i] = cmk((T)0, (T)0);
+#pragma unroll
+            for (int i = 0; i < RREG; ++i) {
+              const int local = first + t.rs + i;
+              if (local >= bend && local < nr) {
+                ++b;
+                bend += P;
+                column();
+              }
+#pragma unroll
+              for (int j = 0; j < NQ; ++j) cfma(k[i], qr[i][j], xr[j]);
+            }
+            add_up(k, first + t.rs, t.rw - t.rs);
+          }
+        }
+        if (!(w & 1)) row_terms();
+        __syncthreads();
+        if (own) {
+          C k = kq[tid];
+          for (int i = 0; i < t.parts; ++i) k = cadd2(k, part[i * t.rows + tid]);
+          C next;
+          if (stage < 3) {
+            ac = stage == 0 ? k : cmk(ac.x + (T)2 * k.x, ac.y + (T)2 * k.y);
+            const T cst = stage < 2 ? (T)0.5 * h : h;
+            next = cmk(yh.x + cst * k.x, yh.y + cst * k.y);
+          } else {
+            const T ix = s6 * (ac.x + k.x), iy = s6 * (ac.y + k.y);
+            double2 v;
+            if constexpr (SPLIT) {
+              dd_add(yh.x, yl.x, ix);
+              dd_add(yh.y, yl.y, iy);
+              v = make_double2((double)yh.x + (double)yl.x, (double)yh.y + (double)yl.y);
+            } else {
+              yh = cmk(yh.x + ix, yh.y + iy);
+              v = yh;
+            }
+            ok = ok && finite2(v);
+            o[(int64_t)step * per + me] = v;
+            next = yh;
+          }
+          xbuf[(size_t)(cur ^ 1) * per + me] = next;
+        }
+        target += t.csize;
+        if (!fe_grid_barrier(t.barrier + 2 * team, target, t.status)) return;
+      }
+    }
+  }
+  if (!ok && t.status) atomicOr(t.status, QSX_ERR_NONFINITE);
+}
+
+// A team of csize CTAs for P pairs and N sites, rreg register rows a warp;
+// false when it does not fit
+template <typename T>
+static bool fe_team_shape(int P, int N, int csize, int rreg, FeTeam* t, size_t* smem) {
+  using C = typename cplx<T>::type;
+  const int per = P * N;
+  t->csize = csize;
+  t->rows = (per + csize - 1) / csize;
+  if (t->rows > FE_TEAM_THREADS) return false;
+  t->rw = (t->rows + FE_TEAM_WARPS - 1) / FE_TEAM_WARPS;
+  t->rs = std::max(0, t->rw - rreg);
+  t->nb = std::min(N, (t->rows + P - 2) / P + 1);
+  t->parts = (N + FE_TEAM_CT - 1) / FE_TEAM_CT;
+  *smem = ((size_t)FE_TEAM_WARPS * t->rs * P + (size_t)t->nb * P +
+           (size_t)(1 + t->parts + N) * t->rows) * sizeof(C);
+  return *smem <= 226 * 1024;
+}
+
+template <typename T>
+static const void* fe_team_entry(int P, int rreg) {
+#define FE_TEAM(NQ)                                                                        \
+  if (P <= 32 * NQ) {                                                                      \
+    if constexpr (sizeof(T) == 4) {                                                        \
+      if (rreg) return (const void*)fe_team_kernel<T, NQ, FE_TEAM_RREG>;                   \
+    }                                                                                      \
+    return rreg ? nullptr : (const void*)fe_team_kernel<T, NQ, 0>;                         \
+  }
+  FE_TEAM(4) FE_TEAM(6) FE_TEAM(9)
+#undef FE_TEAM
+  return nullptr;
+}
+
 // The whole loop of samples whose Q fits one CTA's shared memory, one launch
 // and one CTA a sample: thread e owns the elements e, e + 256, .. of X, its
 // state and stage sums in registers, the stage inputs in shared memory.  For
@@ -368,7 +648,7 @@ __global__ void __launch_bounds__(FE_CTA)
   extern __shared__ __align__(16) unsigned char smraw[];
   const int P = p.P, N = p.N, per = P * N;
   C* sQ = (C*)smraw;               // [P][N][P]
-  C* sR = sQ + (size_t)per * P;    // [N b][N site][N c]
+  C* sR = sQ + (size_t)per * P;    // [N b][N c][N site]
   C* sx = sR + (size_t)N * N * N;  // [2][P N] stage input
   const int64_t s = blockIdx.x;
   for (int i = threadIdx.x; i < per * P; i += FE_CTA) sQ[i] = ((const C*)p.Q)[s * per * P + i];
@@ -417,10 +697,11 @@ __global__ void __launch_bounds__(FE_CTA)
           cfma(k1, q[(size_t)(j + 1) * per], xb[j + 1]);
         }
         if (j < P) cfma(k0, q[(size_t)j * per], xb[j]);
-        const C* ra = sR + (col[i] * N + ka[i]) * N;
-        const C* rb = sR + (col[i] * N + kb[i]) * N;
-        for (int c = 0; c < N; ++c)
-          cfma(k1, in[c * P + row[i]], cmk(ra[c].x + rb[c].x, ra[c].y + rb[c].y));
+        const C* r = sR + col[i] * N * N;
+        for (int c = 0; c < N; ++c) {
+          const C ra = r[c * N + ka[i]], rb = r[c * N + kb[i]];
+          cfma(k1, in[c * P + row[i]], cmk(ra.x + rb.x, ra.y + rb.y));
+        }
         const C k = cadd2(k0, k1);
         if (stage == 0) {
           ac[i] = k;
@@ -604,6 +885,56 @@ extern "C" int qsx_fe_heisenberg_rk4(const void* Q, const void* Ae, const void* 
       if (e != cudaSuccess) return cuda_status(e, "qsx_fe_heisenberg_rk4");
       fe_cta_kernel<T><<<(unsigned)batch, FE_CTA, cta, s>>>(p, (const double2*)y0, y0_stride,
                                                           nsteps, (double2*)out, status);
+      QSX_LAUNCH_CHECK("qsx_fe_heisenberg_rk4");
+      return QSX_OK;
+    }
+    // Q on chip when a team of CTAs holds it, with the team and the register
+    // rows of the shortest loop.  A stage in us, fitted to 11 to 24 sites and 1
+    // to 64 samples: 2.5 for its round trip and 110 ps an element of Q that a
+    // CTA holds; in FP64 3.5 and the multiply-adds at two a clock.  The loop
+    // over the L2 takes its traffic at 6.6 TB/s at least, and 3 us; in FP64
+    // 1.35 times its multiply-adds, and 6 us.
+    const double elements = (double)per * P * (double)batch;
+    const double over_l2 = sizeof(T) == 4 ? 3.0 + elements * sizeof(C) / 6.6e6
+                                          : 6.0 + 1.35 * 4.0 * elements / (2.0 * sms * 1900.0);
+    const double lanes = P <= 128 ? 128 : P <= 192 ? 192 : 288;
+    FeTeam team, pick;
+    size_t tsmem = 0, psmem = 0;
+    const void* pentry = nullptr;
+    double pcost = 0;
+    for (int rreg = 0; rreg <= FE_TEAM_RREG; rreg += FE_TEAM_RREG) {
+      const void* entry = fe_team_entry<T>(P, rreg);
+      for (int c = 1; entry && c <= sms; ++c) {
+        if (!fe_team_shape<T>(P, N, c, rreg, &team, &tsmem)) continue;
+        team.teams = (int)std::min<int64_t>(batch, sms / c);
+        const double cost = (double)((batch + team.teams - 1) / team.teams) *
+                            (sizeof(T) == 4 ? 2.5 + 110e-6 * team.rows * P
+                                            : 3.5 + team.rows * lanes * 4.0 / (2.0 * 1900.0));
+        if (cost < (pentry ? pcost : over_l2)) {
+          pick = team;
+          pentry = entry;
+          psmem = tsmem;
+          pcost = cost;
+        }
+      }
+    }
+    if (pentry) {
+      pick.batch = batch;
+      pick.y0 = (const double2*)y0;
+      pick.y0_stride = y0_stride;
+      pick.nsteps = nsteps;
+      pick.x = yh;                       // two of the five state arrays
+      pick.out = (double2*)out;
+      pick.status = status;
+      pick.barrier = (unsigned*)(yh + 2 * n);
+      e = cudaMemsetAsync(pick.barrier, 0, 2 * sizeof(unsigned) * pick.teams, s);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(pentry, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
+      void* args[] = {&p, &pick};
+      if (e == cudaSuccess)
+        e = cudaLaunchCooperativeKernel(pentry, dim3(pick.teams * pick.csize),
+                                        dim3(FE_TEAM_THREADS), args, psmem, s);
+      if (e != cudaSuccess) return cuda_status(e, "qsx_fe_heisenberg_rk4");
       QSX_LAUNCH_CHECK("qsx_fe_heisenberg_rk4");
       return QSX_OK;
     }

@@ -64,3 +64,16 @@ def test_a_non_finite_state_is_reported():
     with pytest.raises(_native.IntegratorError):
         _native.fe_heisenberg_rk4(Q, z(1, 4, 4), z(1, 4, 4, 4), torch.as_tensor(pairs).cuda(),
                                   torch.ones(24, dtype=torch.complex128, device='cuda'), 3, 1.0)
+
+
+# past one CTA a sample: teams of CTAs with Q on chip (rows in shared memory and
+# in registers, odd and even pair counts, elements of two columns in a CTA, more
+# samples than teams), and the loop over the L2 where no team holds a sample.
+# 32-bit sums of up to 300 terms of that size stay below 1e-5
+@pytest.mark.parametrize('N,S,prec', [(14, 1, 'fp32'), (14, 70, 'fp32'), (16, 20, 'fp32'),
+                                      (17, 5, 'fp32'), (20, 9, 'fp32'), (22, 8, 'fp32'),
+                                      (24, 4, 'fp32'), (26, 1, 'fp32'), (14, 6, 'fp64'),
+                                      (17, 2, 'fp64'), (20, 1, 'fp64'), (22, 1, 'fp64'),
+                                      (24, 1, 'fp64')])
+def test_large_loops_match_numpy(N, S, prec):
+    test_loop_matches_numpy(N, S, prec, True)
