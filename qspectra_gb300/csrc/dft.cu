@@ -4,51 +4,77 @@
 // The reference zero-pads to a symmetric time grid and runs an FFT; padded
 // zeros contribute nothing, so on the FFT frequency grid the result equals
 //   X(f) = dt * sum_n x_n exp(i * sign * (f - rw) * uc * t_n)
-// which this kernel evaluates directly (any grid, e.g. 1024 points in a
-// window).  The twiddle e^{i n Δ} advances by complex rotation and is
-// re-seeded from sincos every 32 samples to bound drift.
+// which these kernels evaluate directly (any grid, e.g. 1024 points in a
+// window), sums of 32 samples at a time by Horner's rule in z = e^{i Delta}
+// (four multiply-adds a sample; a twiddle advanced by rotation takes eight, and
+// the FP64 pipe is the bound), the sums by Horner's rule in z^32, the phase of
+// the first sample from sincos.
 #include "qsx_common.cuh"
 
 namespace qsx {
 
-// grid (ceil(nf / 8), batch), 256 threads: 8 frequencies per CTA, the time
-// samples split into 32 slices, partial sums meet in shared memory (fixed
-// order).
-__global__ void __launch_bounds__(256)
+struct DftPhase {
+  double2 z, z32;   // e^{i w dt}, e^{i 32 w dt}
+};
+
+__device__ __forceinline__ double2 dft_cis(double a) {
+  double2 r;
+  sincos(a, &r.y, &r.x);
+  return r;
+}
+__device__ __forceinline__ DftPhase dft_phase(double wdt) {
+  return {dft_cis(wdt), dft_cis(32.0 * wdt)};
+}
+__device__ __forceinline__ double2 dft_cmul(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
+}
+// a z + x
+__device__ __forceinline__ double2 dft_step(double2 a, double2 z, double2 x) {
+  return make_double2(fma(a.x, z.x, fma(-a.y, z.y, x.x)), fma(a.x, z.y, fma(a.y, z.x, x.y)));
+}
+
+// sum over n < count of x[n stride] z^n
+__device__ __forceinline__ double2 dft_sum(const double2* x, int64_t stride, int count,
+                                           const DftPhase& p) {
+  double2 total = make_double2(0.0, 0.0);
+  for (int b = (count - 1) & ~31; b >= 0; b -= 32) {
+    double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int n = min(count, b + 32) - 1; n >= b; --n) acc = dft_step(acc, p.z, x[n * stride]);
+    total = dft_step(total, p.z32, acc);
+  }
+  return total;
+}
+
+// grid (ceil(nf / 8), batch), 128 threads: 8 frequencies per CTA, each summed
+// over 16 time slices (lane / 8 and the warp pick the slice) that meet in shared
+// memory in a fixed order.  A thread's three sincos cost as much as 60 samples,
+// so 16 slices and not more; 2048 samples at 4095 frequencies took 163 us with
+// rotated twiddles and 32 slices, 86 now.
+constexpr int DFT_SLICES = 16;
+
+__global__ void __launch_bounds__(8 * DFT_SLICES)
     dft_kernel(const double2* __restrict__ x, int nt, double t0, double dt,
                const double* __restrict__ freqs, int nf, double rw, double uc, int sign,
                double2* __restrict__ X) {
-  // 8 frequencies per CTA, each summed over 32 time slices (lane / 8 and the
-  // warp pick the slice), so a spectrum of ~1000 points spreads over ~128
-  // SMs; the slices are added in a fixed order
-  __shared__ double2 part[32][8];
+  __shared__ double2 part[DFT_SLICES][8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int kl = lane & 7, slice = w * 4 + (lane >> 3);
   const int64_t b = blockIdx.y;
   const int k = blockIdx.x * 8 + kl;
   const double wk = k < nf ? (double)sign * (freqs[k] - rw) * uc : 0.0;
-  double sd, cd;
-  sincos(wk * dt, &sd, &cd);
-  const int chunk = (nt + 31) / 32;
+  const DftPhase p = dft_phase(wk * dt);
+  const int chunk = (nt + DFT_SLICES - 1) / DFT_SLICES;
   const int n0 = slice * chunk, n1 = min(nt, n0 + chunk);
-  const double2* xb = x + b * nt;
   double2 acc = make_double2(0.0, 0.0);
-  double2 ph = make_double2(1.0, 0.0);
-  for (int n = n0; n < n1; ++n) {
-    if (((n - n0) & 31) == 0) {   // re-anchor the rotation every 32 steps
-      double s, c;
-      sincos(wk * (t0 + (double)n * dt), &s, &c);
-      ph = make_double2(c, s);
-    }
-    cfma(acc, __ldg(&xb[n]), ph);
-    ph = make_double2(ph.x * cd - ph.y * sd, ph.x * sd + ph.y * cd);
-  }
+  if (n0 < n1)
+    acc = dft_cmul(dft_sum(x + b * nt + n0, 1, n1 - n0, p), dft_cis(wk * (t0 + (double)n0 * dt)));
   part[slice][kl] = acc;
   __syncthreads();
   if (threadIdx.x < 8 && k < nf) {
     double2 t = part[0][kl];
 #pragma unroll
-    for (int i = 1; i < 32; ++i) t = cadd(t, part[i][kl]);
+    for (int i = 1; i < DFT_SLICES; ++i) t = cadd(t, part[i][kl]);
     X[b * nf + k] = cscale(t, dt);
   }
 }
@@ -114,65 +140,41 @@ __global__ void __launch_bounds__(256)
 // t3; any strides) over t1 and t3 in one launch (FP64):
 //   X[k1][b][k3] = dt1 dt3 sum_{n1, n3} x[n1][b][n3]
 //                  exp(i s1 (f1_k1 - rw) uc t1_n1) exp(i s3 (f3_k3 - rw) uc t3_n3),
-// t_n = t0 + n dt on each axis.  CTA (chunk of 8 t3 frequencies, b): first the
+//                  exp(i s1 (f1_k1 - rw) uc t1_n1) exp(i s3 (f3_k3 - rw) uc t3_n3),
+// t_n = t0 + n dt on each axis.  CTA (chunk of F3 t3 frequencies, b): first the
 // t3 transform of every t1 row for those frequencies, into shared memory
-// (Y[n1][8]); then the t1 transform of Y for every t1 frequency.  Each sum
-// advances its twiddle by complex rotation, re-seeded from sincos every 32
-// samples, as dft_kernel does.
-constexpr int DFT2_F3 = 8;
-
+// (Y[n1][F3]); then the t1 transform of Y for every t1 frequency.  The bound is
+// each SM's FP64 pipe, so F3 is the largest of 8, 4, 2 with a CTA for every SM: a
+// 100 x 3 x 100 signal on 199 x 199 frequencies took 652 us in 75 CTAs with
+// rotated twiddles, 173 in 150.
+template <int F3>
 __global__ void __launch_bounds__(256)
     dft2_kernel(const double2* __restrict__ x, int n1, int n3, int64_t s1, int64_t sb,
                 int64_t s3, double t01, double dt1, const double* __restrict__ f1, int nf1,
                 int sign1, double t03, double dt3, const double* __restrict__ f3, int nf3,
                 int sign3, double rw, double uc, double2* __restrict__ X) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  double2* Y = reinterpret_cast<double2*>(smraw);   // [n1][DFT2_F3]
-  const int k3base = blockIdx.x * DFT2_F3;
+  double2* Y = reinterpret_cast<double2*>(smraw);   // [n1][F3]
+  const int kl = threadIdx.x % F3, k = blockIdx.x * F3 + kl;
   const int64_t b = blockIdx.y;
   const int64_t nb = gridDim.y;
   const double2* xb = x + b * sb;
-  // t3 transform: one (n1, k3) sum a thread
-  for (int o = threadIdx.x; o < n1 * DFT2_F3; o += blockDim.x) {
-    const int r = o / DFT2_F3, kl = o % DFT2_F3, k = k3base + kl;
-    double2 acc = make_double2(0.0, 0.0);
-    if (k < nf3) {
-      const double wk = (double)sign3 * (f3[k] - rw) * uc;
-      double sd, cd;
-      sincos(wk * dt3, &sd, &cd);
-      const double2* xr = xb + (int64_t)r * s1;
-      double2 ph = make_double2(1.0, 0.0);
-      for (int n = 0; n < n3; ++n) {
-        if ((n & 31) == 0) {
-          double sn, cn;
-          sincos(wk * (t03 + (double)n * dt3), &sn, &cn);
-          ph = make_double2(cn, sn);
-        }
-        cfma(acc, xr[(int64_t)n * s3], ph);
-        ph = make_double2(ph.x * cd - ph.y * sd, ph.x * sd + ph.y * cd);
-      }
-    }
-    Y[r * DFT2_F3 + kl] = cscale(acc, dt3);
+  // t3 transform: one (n1, k3) sum a thread, the thread's k3 the same in all
+  if (k < nf3) {
+    const double wk = (double)sign3 * (f3[k] - rw) * uc;
+    const DftPhase p = dft_phase(wk * dt3);
+    const double2 first = dft_cis(wk * t03);
+    for (int r = threadIdx.x / F3; r < n1; r += 256 / F3)
+      Y[r * F3 + kl] =
+          cscale(dft_cmul(dft_sum(xb + (int64_t)r * s1, s3, n3, p), first), dt3);
   }
   __syncthreads();
   // t1 transform: one (k1, k3) sum a thread
-  for (int o = threadIdx.x; o < nf1 * DFT2_F3; o += blockDim.x) {
-    const int k1 = o / DFT2_F3, kl = o % DFT2_F3, k = k3base + kl;
-    if (k >= nf3) continue;
+  if (k >= nf3) return;
+  for (int k1 = threadIdx.x / F3; k1 < nf1; k1 += 256 / F3) {
     const double wk = (double)sign1 * (f1[k1] - rw) * uc;
-    double sd, cd;
-    sincos(wk * dt1, &sd, &cd);
-    double2 acc = make_double2(0.0, 0.0), ph = make_double2(1.0, 0.0);
-    for (int n = 0; n < n1; ++n) {
-      if ((n & 31) == 0) {
-        double sn, cn;
-        sincos(wk * (t01 + (double)n * dt1), &sn, &cn);
-        ph = make_double2(cn, sn);
-      }
-      cfma(acc, Y[n * DFT2_F3 + kl], ph);
-      ph = make_double2(ph.x * cd - ph.y * sd, ph.x * sd + ph.y * cd);
-    }
-    X[((int64_t)k1 * nb + b) * nf3 + k] = cscale(acc, dt1);
+    const double2 sum = dft_sum(Y + kl, F3, n1, dft_phase(wk * dt1));
+    X[((int64_t)k1 * nb + b) * nf3 + k] = cscale(dft_cmul(sum, dft_cis(wk * t01)), dt1);
   }
 }
 
@@ -208,7 +210,7 @@ extern "C" int qsx_dft_batched(const double* x, int nt, int64_t batch, double t0
   if (batch == 0) return QSX_OK;
   QSX_CHECK_ARG(x && freqs && X, "qsx_dft_batched: null pointer");
   dim3 grid((unsigned)((nf + 7) / 8), (unsigned)batch);
-  qsx::dft_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
+  qsx::dft_kernel<<<grid, 8 * qsx::DFT_SLICES, 0, (cudaStream_t)stream>>>(
       (const double2*)x, nt, t0, dt, freqs, nf, rw_freq, unit_convert, sign, (double2*)X);
   QSX_LAUNCH_CHECK("qsx_dft_batched");
   return QSX_OK;
@@ -225,18 +227,28 @@ extern "C" int qsx_dft2_batched(const double* x, int n1, int64_t batch, int n3, 
                 "qsx_dft2_batched: signs must be +1 or -1");
   if (batch == 0) return QSX_OK;
   QSX_CHECK_ARG(x && f1 && f3 && X, "qsx_dft2_batched: null pointer");
-  const size_t smem = (size_t)n1 * qsx::DFT2_F3 * sizeof(double2);
-  QSX_CHECK_ARG(smem <= 200 * 1024, "qsx_dft2_batched: n1 = %d too long (at most %d)", n1,
-                (int)(200 * 1024 / (qsx::DFT2_F3 * sizeof(double2))));
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(qsx::dft2_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return qsx::cuda_status(e, "qsx_dft2_batched");
-  }
-  dim3 grid((unsigned)((nf3 + qsx::DFT2_F3 - 1) / qsx::DFT2_F3), (unsigned)batch);
-  qsx::dft2_kernel<<<grid, 256, smem, (cudaStream_t)stream>>>(
-      (const double2*)x, n1, n3, s1, sb, s3, t01, dt1, f1, nf1, sign1, t03, dt3, f3, nf3, sign3,
-      rw_freq, unit_convert, (double2*)X);
-  QSX_LAUNCH_CHECK("qsx_dft2_batched");
-  return QSX_OK;
+  QSX_CHECK_ARG((size_t)n1 * 8 * sizeof(double2) <= 200 * 1024,
+                "qsx_dft2_batched: n1 = %d too long (at most %d)", n1,
+                (int)(200 * 1024 / (8 * sizeof(double2))));
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return qsx::cuda_status(e, "qsx_dft2_batched");
+  auto run = [&](auto kern, int chunk) -> int {
+    const size_t smem = (size_t)n1 * chunk * sizeof(double2);
+    if (smem > 48 * 1024) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return qsx::cuda_status(e, "qsx_dft2_batched");
+    }
+    const dim3 grid((unsigned)((nf3 + chunk - 1) / chunk), (unsigned)batch);
+    kern<<<grid, 256, smem, (cudaStream_t)stream>>>(
+        (const double2*)x, n1, n3, s1, sb, s3, t01, dt1, f1, nf1, sign1, t03, dt3, f3, nf3, sign3,
+        rw_freq, unit_convert, (double2*)X);
+    QSX_LAUNCH_CHECK("qsx_dft2_batched");
+    return QSX_OK;
+  };
+  auto ctas = [&](int chunk) { return (int64_t)((nf3 + chunk - 1) / chunk) * batch; };
+  if (ctas(8) >= sms) return run(qsx::dft2_kernel<8>, 8);
+  // 150 CTAs for 152 SMs are enough
+  return ctas(4) >= sms - sms / 8 ? run(qsx::dft2_kernel<4>, 4) : run(qsx::dft2_kernel<2>, 2);
 }
