@@ -1,4 +1,4 @@
-"""FP64 eigenpairs of small blocks (a warp per matrix, or a thread in large batches) against LAPACK's."""
+"""FP64 eigenpairs of small blocks (a warp or a CTA per matrix, a thread in large batches) against LAPACK's."""
 import numpy as np
 import pytest
 import torch
@@ -32,7 +32,9 @@ def matrices(kind, n, batch):
 @pytest.mark.parametrize('scale', [1.0, 1e-190, 1e200])
 @pytest.mark.parametrize('blocks,batch', [([0, 3], 1), ([0, 4], 5), ([0, 5], 3), ([0, 6], 301),
                                           ([0, 7], 64), ([0, 8], 7), ([0, 1, 8, 12, 14], 33),
-                                          ([0, 3], 600), ([0, 2, 6], 2000)])
+                                          ([0, 3], 600), ([0, 2, 6], 2000),
+                                          ([0, 9], 3), ([0, 1, 16], 5), ([0, 1, 8, 29], 40),
+                                          ([0, 32], 2)])
 def test_eigenpairs(kind, scale, blocks, batch):
     n = blocks[-1]
     A = np.zeros((batch, n, n))
