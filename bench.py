@@ -313,10 +313,11 @@ def heom_ring8(torch, qg, native, samples=64, nsteps=1999):
         e1.record()
         torch.cuda.synchronize()
         out[key] = e0.elapsed_time(e1) * (nsteps / 200)
-    out['form'] = ('library choice (fp32_ms, fp64_ms): the persistent cluster kernel when every '
-                   "sample's cluster is resident at once, else per-stage kernels with a warp "
-                   'per node block; both forced beside, and the per-stage kernels with '
-                   'the node commutators on the tensor cores (variant 3)')
+    out['form'] = ('library choice (fp32_ms, fp64_ms): FP32 the hierarchy on chip, a cluster per '
+                   "sample; FP64 the persistent cluster kernel when every sample's cluster is "
+                   'resident at once, else per-stage kernels with a warp per node block; both '
+                   'forced beside, and the per-stage kernels with the node commutators on the '
+                   'tensor cores (variant 3)')
     k = res['fp64'].shape[0]
     a, b = res['fp32'][:k], res['fp64']
     out['fp32_vs_fp64_rel_err_first_{}_steps'.format(k - 1)] = float(
@@ -493,8 +494,8 @@ def third_order_chain24(torch, qg, samples=256, fp64_samples=8, reps=2, warm=Tru
 def adjoint_fmo7(torch, qg, samples=1024, adam_steps=200, checks=True):
     """Gradient of the absorption misfit (1024 frequencies, 11800-13000 cm^-1)
     of the 7-site model's 1024-sample ensemble (SD 80 cm^-1) w.r.t. 7 site
-    energies, 21 couplings and lambda; 2048 points at 1 fs, checkpoints every
-    64 steps.  Adjoint time vs forward time, FD and autograd checks, Adam."""
+    energies, 21 couplings and lambda; 2048 points at 1 fs, in blocks
+    of 32 steps without checkpoints.  Adjoint time vs forward time, FD and autograd checks, Adam."""
     from qspectra_gb300 import workloads as wl
     from qspectra_gb300.simulate.adjoint import AbsorptionFit
     H7, extra, fwhm = fmo7_inputs()
@@ -583,7 +584,7 @@ def adjoint_fmo7(torch, qg, samples=1024, adam_steps=200, checks=True):
                        'lambda_end': float(theta_fit[-1])}
     return dict({'workload': '7-site Redfield absorption misfit on 1024 frequencies '
                         '(11800-13000 cm^-1), {} disorder samples (SD 80 cm^-1), 2048 x '
-                        '1 fs, checkpoints every 64 steps, 29 parameters'.format(samples),
+                        '1 fs, blocks of 32 steps without checkpoints, 29 parameters'.format(samples),
             'forward_ms': fwd_ms, 'forward_with_graph_ms': fwdg_ms, 'adjoint_ms': bwd_ms,
             'adjoint_over_forward': bwd_ms / fwd_ms}, **out)
 
@@ -624,8 +625,9 @@ def block_roofline(events, bb_flops, bb_ms, fma_peak):
         traffic = ncu_traffic(os.path.join(ROOT, 'profiles', 'block_matrix_tc_fmo7.md'))
         peak, src = measured_tf32_tflops()
         ex = executed / (bb_ms * 1e-3) / 1e12 if bb_ms else None
-        return {'kernel': 'block_matrix_tc_kernel<32> (ee populations, real Hermitian form: '
-                          'K={} step blocked matrices, tcgen05 3xTF32 products in TMEM)'.format(K),
+        return {'kernel': 'block_matrix_tc_kernel<{}> (ee populations, real Hermitian form: '
+                          'K={} step blocked matrices, tcgen05 3xTF32 products, A and the '
+                          'accumulator in TMEM)'.format(kp, K),
                 'bound': 'tensor', 'achieved': bb_achieved, 'peak': peak, 'unit': 'TFLOP/s',
                 'frac': bb_achieved / peak if bb_achieved else None, 'peak_source': src,
                 'executed_tensor_tflops': ex, 'executed_frac': ex / peak if ex else None,
@@ -860,14 +862,16 @@ def our_arm(args):
         return 0
     peak = fma_peak_tflops(torch, _native)
     # the plain FP64 form against the measured FP64 FMA rate.  Its algorithmic
-    # work per step: the step-by-step complex loops in propagator form (one
-    # complex GEMV per RK4 step: ee 49 x 49, eg 7 x 7; 8 flops per complex
-    # multiply-add) and the two one-step propagators (two complex m^3
-    # products each, Paterson-Stockmeyer)
+    # work per step: the ee loop in the real Hermitian form (one real 49 x 49
+    # matrix-vector product per RK4 step, 2 flops per multiply-add), the eg
+    # loop in blocks of 32 steps (32 + m_eg complex rows of m_eg per block, 8
+    # flops per complex multiply-add) and the two one-step propagators (two
+    # m^3 products each, Paterson-Stockmeyer)
     peak64 = fma_peak_tflops(torch, _native, _native.QSX_FP64)
     m_ee, m_eg = len(work.idx_ee), len(work.idx_eg)
     n_dyn, n_abs = len(work.t_dyn) - 1, len(work.t_abs) - 1
-    fp64_flops = 8.0 * S * (n_dyn * m_ee ** 2 + n_abs * m_eg ** 2 + 2 * (m_ee ** 3 + m_eg ** 3))
+    fp64_flops = S * (2.0 * (n_dyn * m_ee ** 2 + 2 * m_ee ** 3)
+                      + 8.0 * (n_abs / 32 * (32 + m_eg) * m_eg + 2 * m_eg ** 3))
     fp64_achieved = fp64_flops / (fp64_ms * 1e-3) / 1e12
     flops_dyn = events['dyn_flops']  # executed form (K-step blocked rows)
     dense_equiv = float(S) * (DYN_TIME - 1) * 49 * 49 * 8  # one 49x49 GEMV per step
@@ -905,9 +909,10 @@ def our_arm(args):
             block_k_real=[{'K': v[0], 'ms': v[1]} for v in block_k_real_timings().values()]),
         'fp64_ms_per_step': fp64_ms, 'speedup_fp32_vs_fp64': fp64_ms / ms,
         'roofline_fp64_form': {
-            'kernel': 'plain FP64 step (complex propagator-form RK4 loops, ee {0} x {0} for {1} '
-                      'steps and eg {2} x {2} for {3} steps, and their one-step propagators; '
-                      'the whole step timed)'.format(m_ee, n_dyn, m_eg, n_abs),
+            'kernel': 'plain FP64 step (propagator-form RK4 loops, ee {0} x {0} real for {1} '
+                      'steps and eg {2} x {2} complex for {3} steps in blocks of 32, and their '
+                      'one-step propagators; the whole step timed)'.format(
+                          m_ee, n_dyn, m_eg, n_abs),
             'bound': 'fp64_fma', 'achieved': fp64_achieved, 'peak': peak64, 'unit': 'TFLOP/s',
             'frac': fp64_achieved / peak64 if peak64 else None, 'flops_per_step': fp64_flops,
             'peak_source': 'measured live by the FMA probe (libqsx_probe.so, FP64 FMA)'},

@@ -219,8 +219,8 @@ def pick_block_k_real(nsteps, m, nselect, max_k=64, tensor_core=None):
     latency-bound part) over ceil(nsteps / K) block-steps, plus the block
     build, nsel m^2 (K-2) for the selected rows and m^3 per product of the
     binary powering.  Where ``tensor_core(K)`` says the tcgen05 build takes
-    K, the build terms weigh 0.6 (its measured time against the CUDA-core
-    build at K = 9).  K need not divide nsteps: the loop runs
+    K, the build terms weigh 0.6 (it takes 0.3 to 0.6 of the CUDA-core build's
+    time; the measurement decides).  K need not divide nsteps: the loop runs
     padded_block_steps(nsteps, K) steps, at most K - 1 more."""
     best, best_cost = 1, None
     for K in range(2, min(max_k, max(int(nsteps), 1)) + 1):
