@@ -179,8 +179,10 @@ __global__ void __launch_bounds__(HS_THREADS, 1) heom_site_kernel(HsP p) {
   const int nrec = p.npcta * p.n_sites;
   for (int i = tid; i <= nrec; i += HS_THREADS) {
     const int l = i / p.n_sites, j = i % p.n_sites;
-    const unsigned self = hs_remote(
-        sx_addr + (unsigned)(min(l, p.npcta - 1) * E * sizeof(float2)), rank);
+    // a missing link reads a node of this CTA, times 0: its own, and the record
+    // of "no site" the first one, as the slots past nloc are never written
+    const unsigned self =
+        hs_remote(sx_addr + (unsigned)((l < nloc ? l : 0) * E * sizeof(float2)), rank);
     HsRecord r = {0.f, 0.f, 0.f, 0.f}, c = r;
     HsLinks k = {self, self};
     if (i < nrec && l < nloc && !several) {
