@@ -377,6 +377,7 @@ __global__ void __launch_bounds__(FE_THREADS, 1) fe_loop_kernel(FeP p, FeLoop l)
 constexpr int FE_TEAM_WARPS = 8, FE_TEAM_THREADS = 32 * FE_TEAM_WARPS;
 constexpr int FE_TEAM_CT = 8;     // columns of a row-term task
 constexpr int FE_TEAM_RREG = 6;   // FP32 rows that a warp can keep in registers
+constexpr int FE_TEAM_NQ[3] = {4, 6, 9};   // terms a lane, of up to 128, 192, 288 pairs
 
 struct FeTeam {
   int64_t batch, y0_stride;
@@ -390,6 +391,14 @@ struct FeTeam {
   unsigned* barrier;     // [teams][2] zeroed: arrivals, abort word
 };
 
+// Elements of the rows in shared memory.  The lanes take 32 NQ terms of a sum
+// over P, those past P times 0: in a row's case the rows after it, in the last
+// one's zeros, since whatever an earlier kernel left may be NaN.
+template <int NQ>
+__host__ __device__ constexpr size_t fe_team_held(int P, int rs) {
+  return rs ? (size_t)FE_TEAM_WARPS * rs * P + (32 * NQ - P) : 0;
+}
+
 template <typename T, int NQ, int RREG>
 __global__ void __launch_bounds__(FE_TEAM_THREADS, 1) fe_team_kernel(FeP p, FeTeam t) {
   using C = typename cplx<T>::type;
@@ -398,8 +407,8 @@ __global__ void __launch_bounds__(FE_TEAM_THREADS, 1) fe_team_kernel(FeP p, FeTe
   constexpr int CT = FE_TEAM_CT;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int P = p.P, N = p.N, per = P * N, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-  C* sQ = (C*)smraw;                                  // [warps][rs][P]
-  C* sx = sQ + (size_t)FE_TEAM_WARPS * t.rs * P;      // [nb P] the columns of the input
+  C* sQ = (C*)smraw;                                  // [warps][rs][P], then zeros
+  C* sx = sQ + fe_team_held<NQ>(P, t.rs);             // [nb P] the columns of the input
   C* kq = sx + (size_t)t.nb * P;                      // [rows] column terms
   C* part = kq + t.rows;                              // [parts][rows] row terms
   const int team = blockIdx.x / t.csize;
@@ -417,6 +426,9 @@ __global__ void __launch_bounds__(FE_TEAM_THREADS, 1) fe_team_kernel(FeP p, FeTe
   const T h = (T)p.h, s6 = h / (T)6;
   unsigned target = 0;
   bool ok = true;
+  if (t.rs)
+    for (int e = FE_TEAM_WARPS * t.rs * P + tid; sQ + e < sx; e += FE_TEAM_THREADS)
+      sQ[e] = cmk((T)0, (T)0);
   for (int64_t s = team; s < t.batch; s += t.teams) {
     const C* Qg = (const C*)p.Q + s * (int64_t)per * P + rho0;
     const C* Rg = (const C*)p.R + s * (int64_t)N * N * N;
@@ -612,7 +624,10 @@ static bool fe_team_shape(int P, int N, int csize, int rreg, FeTeam* t, size_t* 
   t->rs = std::max(0, t->rw - rreg);
   t->nb = std::min(N, (t->rows + P - 2) / P + 1);
   t->parts = (N + FE_TEAM_CT - 1) / FE_TEAM_CT;
-  *smem = ((size_t)FE_TEAM_WARPS * t->rs * P + (size_t)t->nb * P +
+  const size_t held = P <= 32 * FE_TEAM_NQ[0]   ? fe_team_held<FE_TEAM_NQ[0]>(P, t->rs)
+                      : P <= 32 * FE_TEAM_NQ[1] ? fe_team_held<FE_TEAM_NQ[1]>(P, t->rs)
+                                                : fe_team_held<FE_TEAM_NQ[2]>(P, t->rs);
+  *smem = (held + (size_t)t->nb * P +
            (size_t)(1 + t->parts + N) * t->rows) * sizeof(C);
   return *smem <= 226 * 1024;
 }
@@ -626,7 +641,7 @@ static const void* fe_team_entry(int P, int rreg) {
     }                                                                                      \
     return rreg ? nullptr : (const void*)fe_team_kernel<T, NQ, 0>;                         \
   }
-  FE_TEAM(4) FE_TEAM(6) FE_TEAM(9)
+  FE_TEAM(FE_TEAM_NQ[0]) FE_TEAM(FE_TEAM_NQ[1]) FE_TEAM(FE_TEAM_NQ[2])
 #undef FE_TEAM
   return nullptr;
 }

@@ -7,6 +7,7 @@ import torch
 import qspectra_gb300 as qg
 from conftest import rel_err
 from qspectra_gb300 import _native
+from test_gpu_fe_heisenberg import test_loop_matches_numpy as compare_fe_loop
 from test_gpu_heom_site import tables
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +40,14 @@ def test_hierarchy_on_chip(n, level, S, fill_with_nan):
     fill_with_nan()
     x = run(_native.QSX_FP32, 0)
     assert rel_err(x, run(_native.QSX_FP64, 1)) < 1e-5
+
+
+# teams of CTAs whose last rows end at unwritten columns of X or at the sums, by
+# the plan on 152 SMs: P = 28 to 55 of the 128 terms that the lanes take
+@pytest.mark.parametrize('N,S,prec', [(8, 4, 'fp64'), (8, 5, 'fp64'), (8, 10, 'fp64'),
+                                      (8, 15, 'fp64'), (9, 3, 'fp64'), (9, 7, 'fp64'),
+                                      (10, 8, 'fp64'), (11, 2, 'fp64'), (11, 4, 'fp64'),
+                                      (11, 2, 'fp32'), (11, 4, 'fp32')])
+def test_two_exciton_team(N, S, prec, fill_with_nan):
+    fill_with_nan()
+    compare_fe_loop(N, S, prec, True)
