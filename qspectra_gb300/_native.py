@@ -9,6 +9,8 @@ import os
 
 import numpy as np
 import torch
+from torch.autograd.forward_ad import unpack_dual
+from torch.utils._python_dispatch import _get_current_dispatch_mode
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, '_lib', 'libqsx.so')
@@ -240,6 +242,18 @@ def _check(status, what):
 def _stream():
     # the handle alone: building a Stream object costs microseconds a launch
     return _c_vp(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+
+def plain(*tensors):
+    """Whether kernels may read these tensors by their pointers: ordinary
+    tensors, and no transform (vmap, forward-mode or functorch), tracer or
+    dispatch mode that has to see the operations on them."""
+    if (torch.compiler.is_compiling() or torch.jit.is_tracing()
+            or torch._C._are_functorch_transforms_active()
+            or _get_current_dispatch_mode() is not None):
+        return False
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter)
+               and unpack_dual(t).tangent is None for t in tensors)
 
 
 def _p(t):

@@ -103,40 +103,78 @@ class SymmetricEigh(torch.autograd.Function):
 class EgGenerator(torch.autograd.Function):
     """Heisenberg 'eg' generators L of rotating-frame Hamiltonians H (S, N, N)
     and a reorganisation energy, N <= 16: one kernel after the eigensolve and
-    one backward (qsx_eg_generator, qsx_eg_generator_adjoint)."""
+    one backward (qsx_eg_generator, qsx_eg_generator_adjoint).  A backward
+    that is to be differentiated itself goes through the array form."""
 
     @staticmethod
     def forward(ctx, H, lam, temperature, cutoff_freq, unit_convert, matsubara_cutoff):
-        H = H.detach().contiguous()
-        E, U = _native.eigh(H, [0, H.shape[-1]])
-        L, c0, d0 = _native.eg_generator(H, E, U, lam.detach(), temperature, cutoff_freq,
-                                         matsubara_cutoff, unit_convert)
-        ctx.save_for_backward(E, U, c0, d0, lam)
-        ctx.unit_convert = unit_convert
+        Hc = H.detach().contiguous()
+        E, U = _native.eigh(Hc, [0, H.shape[-1]])
+        L, c0, d0 = _native.eg_generator(Hc, E, U, lam.detach().resolve_neg(), temperature,
+                                         cutoff_freq, matsubara_cutoff, unit_convert)
+        ctx.save_for_backward(H, lam, E, U, c0, d0)
+        ctx.args = (temperature, cutoff_freq, unit_convert, matsubara_cutoff)
         return L
 
     @staticmethod
     def backward(ctx, g):
-        E, U, c0, d0, lam = ctx.saved_tensors
-        gH, glam = _native.eg_generator_adjoint(E, U, lam, ctx.unit_convert, c0, d0, g)
-        return gH, glam.sum().reshape(lam.shape), None, None, None, None
+        H, lam, E, U, c0, d0 = ctx.saved_tensors
+        if torch.is_grad_enabled():   # create_graph
+            T, gam, uc, K = ctx.args
+            L = _generator_arrays(H, lam, uc, SymmetricEigh.apply,
+                                  lambda x: _debye_arrays(x, lam, T, gam, K))
+            need = [t for t, n in zip((H, lam), ctx.needs_input_grad) if n]
+            got = iter(torch.autograd.grad(L, need, g, create_graph=True))
+            gH, glam = (next(got) if n else None for n in ctx.needs_input_grad[:2])
+        else:
+            # autograd may hand over a conjugate view, the kernel reads the memory
+            gH, glam = _native.eg_generator_adjoint(E, U, lam.resolve_neg(), ctx.args[2], c0, d0,
+                                                    g.resolve_conj())
+            glam = glam.sum().reshape(lam.shape)
+        return gH, glam, None, None, None, None
 
 
 class RK4Step(torch.autograd.Function):
-    """D = P - I of one RK4 step of L (S, N, N), N <= 16, one kernel each way."""
+    """D = P - I of one RK4 step of L (S, N, N), N <= 16, one kernel each way;
+    a backward that is to be differentiated itself goes through the array
+    form.  L is the caller's to keep unchanged until then."""
 
     @staticmethod
     def forward(ctx, L, h):
-        # a copy: the caller may reuse L's memory before the backward pass
-        L = L.detach().clone(memory_format=torch.contiguous_format)
         ctx.save_for_backward(L)
         ctx.h = h
-        return _native.rk4_step(L, h)
+        return _native.rk4_step(L.detach(), h)
 
     @staticmethod
     def backward(ctx, g):
         (L,) = ctx.saved_tensors
-        return _native.rk4_step_adjoint(L, g, ctx.h), None
+        if torch.is_grad_enabled():   # create_graph
+            return torch.autograd.grad(_rk4_step_arrays(L, ctx.h), L, g, create_graph=True)[0], None
+        return _native.rk4_step_adjoint(L, g.resolve_conj(), ctx.h), None
+
+
+def _debye_arrays(x, lam, temperature, cutoff_freq, matsubara_cutoff):
+    """lam C_unit(x) (see _debye_unit) by array operations, to be
+    differentiated any number of times."""
+    T, gam = float(temperature), float(cutoff_freq)
+    nu = 2 * np.pi * T * torch.arange(1, matsubara_cutoff, dtype=torch.float64, device=x.device)
+    w = nu / (nu ** 2 - gam ** 2)
+    ix = 1j * x.to(torch.complex128)
+    val = gam * ((1.0 / np.tan(gam / (2 * T)) - 1j) / (gam - ix)
+                 + 4 * T * (w / (nu - ix[..., None])).sum(-1))
+    # x = 0: the reference's limit, with the slope of the sum
+    return lam * (val + torch.where(x == 0, 2 * T / gam - 1j - val.detach(), 0.0))
+
+
+def _generator_arrays(H, lam, unit_convert, eigh, corr):
+    E, U = eigh(H)
+    x = E[:, None, :] - E[:, :, None]                 # x[c][d] = E_d - E_c
+    C = corr(x)
+    Uc = U.to(torch.complex128)
+    W = (U * U).to(torch.complex128) @ C              # W[a][d] = sum_c U[a][c]^2 C[c][d]
+    G = unit_convert * ((W * Uc) @ Uc.transpose(1, 2))
+    A = G + 1j * unit_convert * H.to(torch.complex128)
+    return -A.transpose(1, 2)
 
 
 def eg_heisenberg_generator(H1, lam, temperature, cutoff_freq, rw_freq, unit_convert,
@@ -155,27 +193,29 @@ def eg_heisenberg_generator(H1, lam, temperature, cutoff_freq, rw_freq, unit_con
     H = H1 - rw_freq * eye
     if (eigh is None and H.is_cuda and H.dtype == torch.float64 and H.dim() == 3
             and N <= _native.FIT_MAX and isinstance(lam, torch.Tensor) and lam.is_cuda
-            and lam.dtype == torch.float64 and lam.numel() == 1):
+            and lam.dtype == torch.float64 and lam.numel() == 1 and _native.plain(H, lam)):
         return EgGenerator.apply(H, lam, float(temperature), float(cutoff_freq), unit_convert,
                                  matsubara_cutoff)
-    E, U = (eigh or SymmetricEigh.apply)(H)
-    x = E[:, None, :] - E[:, :, None]                 # x[c][d] = E_d - E_c
-    C = DebyeCorr.apply(x, lam, temperature, cutoff_freq, matsubara_cutoff)
-    Uc = U.to(torch.complex128)
-    W = (U * U).to(torch.complex128) @ C              # W[a][d] = sum_c U[a][c]^2 C[c][d]
-    G = unit_convert * ((W * Uc) @ Uc.transpose(1, 2))
-    A = G + 1j * unit_convert * H.to(torch.complex128)
-    return -A.transpose(1, 2)
+    return _generator_arrays(
+        H, lam, unit_convert, eigh or SymmetricEigh.apply,
+        lambda x: DebyeCorr.apply(x, lam, temperature, cutoff_freq, matsubara_cutoff))
+
+
+def _rk4_step_arrays(L, h):
+    A = h * L
+    A2 = A @ A
+    return A + 0.5 * A2 + A2 @ (A / 6 + A2 / 24)
 
 
 def rk4_step_minus_identity(L, h):
     """D = P - I, P = sum_{k<=4} (hL)^k / k! (Paterson-Stockmeyer form)."""
     if (L.is_cuda and L.dtype == torch.complex128 and L.dim() == 3
-            and L.shape[-2] == L.shape[-1] <= _native.FIT_MAX and isinstance(h, (int, float))):
-        return RK4Step.apply(L, h)
-    A = h * L
-    A2 = A @ A
-    return A + 0.5 * A2 + A2 @ (A / 6 + A2 / 24)
+            and L.shape[-2] == L.shape[-1] <= _native.FIT_MAX and isinstance(h, (int, float))
+            and _native.plain(L)):
+        # a copy: the caller may reuse L's memory before the backward pass, and
+        # a conjugate view becomes the values themselves
+        return RK4Step.apply(L.clone(memory_format=torch.contiguous_format), h)
+    return _rk4_step_arrays(L, h)
 
 
 # ------------------------------------------------------------- time loop
@@ -185,7 +225,7 @@ class ProjectedMeanRK4(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, D, y0, c, nsteps, ck_every):
-        D = D.detach().contiguous()
+        D = D.detach().contiguous().resolve_conj()
         S, m, _ = D.shape
         out = _native.rk4(D, y0, nsteps, 1, proj=c[None], per_sample=False, mean=True,
                           precision=_native.QSX_FP64)
@@ -199,7 +239,7 @@ class ProjectedMeanRK4(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         D, y0, c = ctx.saved_tensors
-        gradD = _native.rk4_mean_adjoint(D, y0, ctx.ck_every, ctx.nsteps, c, g.contiguous(),
+        gradD = _native.rk4_mean_adjoint(D, y0, ctx.ck_every, ctx.nsteps, c, g.resolve_conj(),
                                          1.0 / D.shape[0])
         return gradD, None, None, None, None
 
@@ -222,7 +262,7 @@ class Dft(torch.autograd.Function):
         f = f.numpy()
         df = (f[-1] - f[0]) / (len(f) - 1)
         t = torch.arange(nt, dtype=torch.float64) * dt
-        gx = _native.dft(g.contiguous(), f[0] - rw, df, t, 0.0, uc, -1) * (dt / df)
+        gx = _native.dft(g.contiguous().resolve_conj(), f[0] - rw, df, t, 0.0, uc, -1) * (dt / df)
         return gx, None, None, None, None
 
 
