@@ -64,7 +64,10 @@ class SampleBatch:
         ham = self.model.hamiltonian
         base = _native.upload(ham.H(subspace), torch.float64)
         n = base.shape[0]
-        if 'e' in subspace:
+        # one kernel, unless something has to see the operations on the offsets
+        off = self.offsets
+        kernel = _native.plain(off) and not (off.requires_grad and torch.is_grad_enabled())
+        if 'e' in subspace and kernel:
             sl = hilbert_subspace_index('e', subspace, ham.n_sites)
             H = _native.disordered_hamiltonians(
                 base, self.offsets.expand(self.size, ham.n_sites).contiguous(), sl.start)
@@ -73,7 +76,7 @@ class SampleBatch:
         if 'f' in subspace:
             sl = hilbert_subspace_index('f', subspace, ham.n_sites)
             ii, jj = _native.upload(np.array(pair_sites(ham.n_sites)))
-            H.diagonal(dim1=1, dim2=2)[:, sl] += self.offsets[:, ii] + self.offsets[:, jj]
+            H.diagonal(dim1=1, dim2=2)[:, sl].add_(off[:, ii] + off[:, jj])
         return H.contiguous()
 
 
