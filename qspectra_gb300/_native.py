@@ -288,21 +288,6 @@ def upload(values, dtype=None, device='cuda'):
     return t.pin_memory().to(device, non_blocking=True)
 
 
-class Ready:
-    """The end of the work so far on the current stream: what an object that
-    outlives a call was filled by.  ``wait`` lets the work that follows on
-    another stream begin after it (a graph captures nothing that is not done)."""
-
-    def __init__(self):
-        self.stream = _stream().value
-        self.event = torch.cuda.Event()
-        self.event.record()
-
-    def wait(self):
-        if _stream().value != self.stream and not torch.cuda.is_current_stream_capturing():
-            self.event.wait()
-
-
 def check_later(later):
     """Read the status words that calls given ``later=`` left in it, with one
     synchronisation, and raise what the first of them to fail would have."""
@@ -1200,7 +1185,6 @@ class CsrMap:
         _check(load().qsx_csr_map_batched(_p(xb), n_in, xb.shape[0], _p(self.rowptr),
                                           _p(self.cols), _p(self.vals), n_out, _p(out),
                                           _stream()), 'qsx_csr_map_batched')
-        self._ready = Ready() if data.is_cuda else None
         return out.reshape(tuple(lead) + (n_out,))
 
 
@@ -1208,7 +1192,6 @@ def rk4_adjoint(D, checkpoints, ck_every, nsteps, c, g, scale, want_y0=False):
     """grad of sum_n Re(conj(g_n) x_n) w.r.t. D (and y0) for the mean projected
     RK4 loop (qsx_rk4_adjoint_batched).  D (B, m, m) complex128; checkpoints
     (B, nck, m) complex128; c (m,), g (nsteps+1,) complex128."""
-        self._ready.wait()
     require_gpu()
     _need(D, torch.complex128, 'D', 3)
     _need(checkpoints, torch.complex128, 'checkpoints', 3)
