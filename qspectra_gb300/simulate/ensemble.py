@@ -70,9 +70,12 @@ class SampleBatch:
         if 'e' in subspace and kernel:
             sl = hilbert_subspace_index('e', subspace, ham.n_sites)
             H = _native.disordered_hamiltonians(
-                base, self.offsets.expand(self.size, ham.n_sites).contiguous(), sl.start)
+                base, off.expand(self.size, ham.n_sites).contiguous().resolve_neg(), sl.start)
         else:
             H = base.expand(self.size, n, n).clone()
+            if 'e' in subspace:
+                sl = hilbert_subspace_index('e', subspace, ham.n_sites)
+                H.diagonal(dim1=1, dim2=2)[:, sl].add_(off)
         if 'f' in subspace:
             sl = hilbert_subspace_index('f', subspace, ham.n_sites)
             ii, jj = _native.upload(np.array(pair_sites(ham.n_sites)))
