@@ -288,6 +288,21 @@ def upload(values, dtype=None, device='cuda'):
     return t.pin_memory().to(device, non_blocking=True)
 
 
+class Ready:
+    """The end of the work so far on the current stream: what an object that
+    outlives a call was filled by.  ``wait`` lets the work that follows on
+    another stream begin after it (a graph captures nothing that is not done)."""
+
+    def __init__(self):
+        self.stream = _stream().value
+        self.event = torch.cuda.Event()
+        self.event.record()
+
+    def wait(self):
+        if _stream().value != self.stream and not torch.cuda.is_current_stream_capturing():
+            self.event.wait()
+
+
 def check_later(later):
     """Read the status words that calls given ``later=`` left in it, with one
     synchronisation, and raise what the first of them to fail would have."""
@@ -1172,6 +1187,7 @@ class CsrMap:
         self.vals = data[:16 * n].view(torch.complex128)
         self.cols = data[16 * n:20 * n].view(torch.int32)
         self.rowptr = data[20 * n:].view(torch.int32)
+        self._ready = Ready() if data.is_cuda else None
 
     def __call__(self, x):
         """x (..., n_in) complex128 CUDA -> (..., n_out)."""
@@ -1179,6 +1195,7 @@ class CsrMap:
         n_out, n_in = self.shape
         if x.shape[-1] != n_in:
             raise ValueError('map takes {} components (got {})'.format(n_in, x.shape[-1]))
+        self._ready.wait()
         lead = x.shape[:-1]
         xb = x.to(torch.complex128).reshape(-1, n_in).contiguous()
         out = torch.empty((xb.shape[0], n_out), dtype=torch.complex128, device=x.device)

@@ -59,9 +59,11 @@ class SampleBatch:
         else:
             self.offsets = torch.as_tensor(np.asarray(offsets, float),
                                            dtype=torch.float64).cuda()
+        self._ready = _native.Ready()      # the draws are a kernel of this stream
 
     def H(self, subspace):
         ham = self.model.hamiltonian
+        self._ready.wait()
         base = _native.upload(ham.H(subspace), torch.float64)
         n = base.shape[0]
         # one kernel, unless something has to see the operations on the offsets

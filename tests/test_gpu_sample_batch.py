@@ -1,9 +1,10 @@
-"""The Hamiltonians of disorder samples: what the offsets may be."""
+"""The Hamiltonians of disorder samples: what the offsets may be, and streams."""
 import numpy as np
 import pytest
 import torch
 
 import qspectra_gb300 as qg
+from qspectra_gb300 import _native
 from qspectra_gb300 import workloads as wl
 from qspectra_gb300.simulate.ensemble import SampleBatch
 
@@ -54,3 +55,20 @@ def test_every_form_of_offsets(subspace, form):
                  for i in range(4)]]
         want = np.einsum('sab,niab->si', w.cpu().numpy(), np.array(want))
         np.testing.assert_allclose(t.grad.cpu().numpy(), want, rtol=1e-13, atol=1e-13)
+
+
+def test_objects_made_on_a_busy_stream_serve_another():
+    m = model(disorder=100.0, random_seed=3)
+    off = m.hamiltonian.disorder_offsets(64)
+    dense = np.random.RandomState(1).randn(40, 30) + 0j
+    x = torch.ones(3, 30, dtype=torch.complex128, device='cuda')
+    torch.cuda.synchronize()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(100_000_000)      # about 50 ms
+        batch, table = SampleBatch(m, 64), _native.CsrMap(dense)
+    with torch.cuda.stream(b):
+        H, y = batch.H('e'), table(x)
+        H, y = H.cpu().numpy(), y.cpu().numpy()
+    np.testing.assert_allclose(H, expected(m, off, 'e'), rtol=1e-13)
+    np.testing.assert_allclose(y, np.repeat(dense.sum(1)[None], 3, 0), rtol=1e-13)
