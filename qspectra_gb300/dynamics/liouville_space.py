@@ -106,17 +106,29 @@ class LinearMap:
         """The matrix on the GPU."""
         if self._matrix is None:
             self._matrix = torch.as_tensor(self._host, device=_device())
+            self._version = self._matrix._version
         return self._matrix
+
+    @matrix.setter
+    def matrix(self, value):
+        self._matrix, self._version, self._host = value, value._version, None
 
     @property
     def shape(self):
-        return self._host.shape
+        return tuple((self._host if self._matrix is None else self._matrix).shape)
+
+    def _on_host(self):
+        """The matrix on the host, while the one on the GPU is the same."""
+        if self._matrix is not None and self._matrix._version != self._version:
+            self._host = None
+        return self._host
 
     def __call__(self, state):
-        if (not isinstance(state, torch.Tensor) and np.ndim(state) == 1
-                and self._host.size <= self.HOST_MAX):
-            y = self._host @ np.asarray(state, dtype=complex)
-            return y[..., 0] if self.scalar else y
+        if not isinstance(state, torch.Tensor) and np.ndim(state) == 1:
+            m = self._on_host()
+            if m is not None and m.size <= self.HOST_MAX:
+                y = m @ np.asarray(state, dtype=complex)
+                return y[0, ...] if self.scalar else y     # a 0-d array, as from the GPU
         x, is_tensor = _as_device(state)
         y = x @ self.matrix.T
         if self.scalar:
