@@ -92,12 +92,34 @@ __device__ __forceinline__ void col_rank2(double* __restrict__ x, int ld,
 
 constexpr int TQ_THREADS = 320;
 
+// The exponent of a matrix's largest element, which the reduction divides out:
+// the square of no element that matters then leaves the range.  0 for a matrix
+// of zeros and for one that is not finite (the eigenvalues report that).
+__device__ __forceinline__ int scale_of(double top) {
+  return top > 0.0 && isfinite(top) ? ilogb(top) : 0;
+}
+__device__ __forceinline__ double larger(double top, double v) {
+  return isfinite(v) ? fmax(top, fabs(v)) : INFINITY;
+}
+
+// The reflector of a column (x0, rest), rest the sum of the squares below x0:
+// summed by itself, since |x|^2 - x0^2 loses what lies 1e-8 below x0.
+struct Reflector {
+  double alpha, v0, tau;   // tau = 0: the column is done as it is
+};
+__device__ __forceinline__ Reflector reflector(double x0, double rest) {
+  if (rest == 0.0) return {x0, x0, 0.0};   // (NaN goes on and is reported)
+  const double alpha = -copysign(sqrt(fma(x0, x0, rest)), x0), v0 = x0 - alpha;
+  return {alpha, v0, 2.0 / fma(v0, v0, rest)};
+}
+
 // ---- A. Householder tridiagonalisation: one CTA per matrix.  Writes the
-// diagonal and sub-diagonal to de[b] = {d[0..n), e[0..n)} and keeps, in the
-// work matrix W, each reflector v_k in row k right of the diagonal with
-// tau_k on the diagonal.
+// diagonal and sub-diagonal of A / 2^ex to de[b] = {d[0..n), e[0..n)}, ex to
+// expo[b], and keeps, in the work matrix W, each reflector v_k in row k right of
+// the diagonal with tau_k on the diagonal.
 __global__ void __launch_bounds__(TQ_THREADS, 2)
-    eigh_tridiag_kernel(const double* __restrict__ A, int n, double* W, double* de) {
+    eigh_tridiag_kernel(const double* __restrict__ A, int n, double* W, double* de,
+                        double* expo) {
   extern __shared__ __align__(16) double sm[];
   double* v = sm;          // [n] Householder vector
   double* w = v + n;       // [n]
@@ -109,7 +131,15 @@ __global__ void __launch_bounds__(TQ_THREADS, 2)
   double* Wm = W + b * nn;
   double* d = de + b * 2 * (int64_t)n;
   double* e = d + n;
-  for (int64_t i = tid; i < nn; i += bd) Wm[i] = a[i];
+  double top = 0.0;
+  for (int64_t i = tid; i < nn; i += bd) top = larger(top, a[i]);
+  for (int o = 16; o; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if ((tid & 31) == 0) red[tid >> 5] = top;
+  __syncthreads();
+  for (int i = 0; i < bd >> 5; ++i) top = fmax(top, red[i]);
+  const int ex = scale_of(top);
+  if (tid == 0) expo[b] = (double)ex;
+  for (int64_t i = tid; i < nn; i += bd) Wm[i] = scalbn(a[i], -ex);
   __syncthreads();
   for (int k = 0; k < n - 2; ++k) {
     const int m = n - k - 1;
@@ -118,21 +148,18 @@ __global__ void __launch_bounds__(TQ_THREADS, 2)
     for (int i = tid; i < m; i += bd) {
       const double x = rowk[i];
       v[i] = x;
-      part += x * x;
+      if (i) part += x * x;
     }
-    const double sigma = block_sum(part, red);
-    const double x0 = v[0];
-    double tau = 0.0;
-    if (tid == 0) d[k] = Wm[(int64_t)k * n + k];
-    if (sigma - x0 * x0 > 0.0) {
-      const double alpha = -copysign(sqrt(sigma), x0);
-      const double v0 = x0 - alpha;
-      tau = 2.0 / (sigma - x0 * x0 + v0 * v0);
+    const double rest = block_sum(part, red);
+    const Reflector f = reflector(v[0], rest);
+    const double tau = f.tau;
+    if (tid == 0) {
+      d[k] = Wm[(int64_t)k * n + k];
+      e[k] = f.alpha;
+    }
+    if (tau != 0.0) {
       __syncthreads();
-      if (tid == 0) {
-        v[0] = v0;
-        e[k] = alpha;
-      }
+      if (tid == 0) v[0] = f.v0;
       __syncthreads();
       double* B = Wm + (int64_t)(k + 1) * n + k + 1;
       // p = tau B v (B symmetric: column r read across threads)
@@ -146,8 +173,6 @@ __global__ void __launch_bounds__(TQ_THREADS, 2)
       for (int r = tid; r < m; r += bd) w[r] -= K * v[r];
       __syncthreads();
       for (int c = tid; c < m; c += bd) col_rank2(B + c, n, v, w, w[c], v[c], m);
-    } else {
-      if (tid == 0) e[k] = x0;
     }
     __syncthreads();
     for (int i = tid; i < m; i += bd) Wm[(int64_t)k * n + k + 1 + i] = tau != 0.0 ? v[i] : 0.0;
@@ -207,7 +232,8 @@ __device__ __forceinline__ double warp_dot(const double* x, const double* y, int
 }
 
 __global__ void __launch_bounds__(TC_THREADS)
-    eigh_tridiag_cluster_kernel(const double* __restrict__ A, int n, int c, double* W, double* de) {
+    eigh_tridiag_cluster_kernel(const double* __restrict__ A, int n, int c, double* W, double* de,
+                                double* expo) {
   extern __shared__ __align__(16) double sm[];
   const int ld = tri_ld(n), cols = (n + c - 1) / c;
   double* B = sm;                        // [cols][ld], column lc is matrix column lc c + rank
@@ -217,6 +243,7 @@ __global__ void __launch_bounds__(TC_THREADS)
   double* w = vbuf + 2 * n;              // [n] p
   double* head = w + n;                  // [2]
   double* sv = head + 2;                 // [3] v_0, tau and K of this step
+  __shared__ double tops[TC_THREADS / 32], ctop[TC_MAX_CLUSTER];
   const int tid = threadIdx.x;
   const int rank = (int)cluster_rank();
   const int64_t b = blockIdx.x / c, nn = (int64_t)n * n;
@@ -224,34 +251,47 @@ __global__ void __launch_bounds__(TC_THREADS)
   double* Wm = W + b * nn;
   double* d = de + b * 2 * (int64_t)n;
   double* e = d + n;
+  double top = 0.0;
   for (int64_t i = tid; i < (int64_t)cols * n; i += TC_THREADS) {
     // symmetric: row j of A is column j, read along the row
     const int lc = (int)(i / n), r = (int)(i % n), j = lc * c + rank;
-    if (j < n) B[(size_t)lc * ld + r] = a[(int64_t)j * n + r];
+    if (j >= n) continue;
+    const double v = a[(int64_t)j * n + r];
+    B[(size_t)lc * ld + r] = v;
+    top = larger(top, v);
   }
+  for (int o = 16; o; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+  if ((tid & 31) == 0) tops[tid >> 5] = top;
   __syncthreads();
   cluster_barrier();   // every CTA of the cluster runs before remote stores
+  if (tid < c) {
+    for (int i = 0; i < TC_THREADS / 32; ++i) top = fmax(top, tops[i]);
+    store_remote(ctop + rank, tid, top);
+  }
+  cluster_barrier();
+  top = ctop[0];
+  for (int i = 1; i < c; ++i) top = fmax(top, ctop[i]);
+  const int ex = scale_of(top);
+  if (rank == 0 && tid == 0) expo[b] = (double)ex;
+  for (int64_t i = tid; i < (int64_t)cols * n; i += TC_THREADS) {
+    const int lc = (int)(i / n), r = (int)(i % n);
+    if (lc * c + rank < n) B[(size_t)lc * ld + r] = scalbn(B[(size_t)lc * ld + r], -ex);
+  }
+  __syncthreads();
   for (int k = 0; k < n - 2; ++k) {
     double* v = vbuf + (k & 1) * n;
     if (rank == k % c) {
       // one warp: more of them would only queue for the FP64 pipe
       const double* x = B + (size_t)(k / c) * ld;
       if (tid < 32) {
-        const double sigma = warp_dot(x, x, k + 1 + tid, n);
-        const double x0 = x[k + 1];
-        double tau = 0.0, v0 = x0, alpha = x0;
-        if (sigma - x0 * x0 > 0.0) {
-          alpha = -copysign(sqrt(sigma), x0);
-          v0 = x0 - alpha;
-          tau = 2.0 / (sigma - x0 * x0 + v0 * v0);
-        }
-        if (tid < c) store_remote(head + (k & 1), tid, tau);
+        const Reflector f = reflector(x[k + 1], warp_dot(x, x, k + 2 + tid, n));
+        if (tid < c) store_remote(head + (k & 1), tid, f.tau);
         if (tid == 0) {
-          sv[0] = v0;
-          sv[1] = tau;
+          sv[0] = f.v0;
+          sv[1] = f.tau;
           d[k] = x[k];
-          e[k] = alpha;
-          Wm[(int64_t)k * n + k] = tau;
+          e[k] = f.alpha;
+          Wm[(int64_t)k * n + k] = f.tau;
         }
       }
       __syncthreads();
@@ -639,8 +679,9 @@ constexpr int BT_THREADS = 512;
 
 __global__ void __launch_bounds__(BT_THREADS)
     eigh_backtransform_kernel(const double* __restrict__ W, const double* __restrict__ ws,
-                              int n, int cols, int parts, const double* __restrict__ Z,
-                              double* __restrict__ E, double* __restrict__ U) {
+                              const double* __restrict__ expo, int n, int cols, int parts,
+                              const double* __restrict__ Z, double* __restrict__ E,
+                              double* __restrict__ U) {
   extern __shared__ __align__(16) double sm[];
   const int ld = tri_ld(n);
   double* z = sm;                       // [cols][ld]
@@ -683,7 +724,7 @@ __global__ void __launch_bounds__(BT_THREADS)
     }
     __syncthreads();
   }
-  for (int i = tid; i < nc; i += blockDim.x) E[b * n + c0 + i] = ws[b * n + c0 + i];
+  for (int i = tid; i < nc; i += blockDim.x) E[b * n + c0 + i] = scalbn(ws[b * n + c0 + i], (int)expo[b]);
   for (int64_t i = tid; i < (int64_t)n * nc; i += blockDim.x) {
     const int r = (int)(i / nc), c = (int)(i % nc);
     U[b * nn + (int64_t)r * n + c0 + c] = z[(size_t)c * ld + r];
@@ -697,10 +738,10 @@ using namespace qsx;
 extern "C" size_t qsx_eigh_large_workspace_bytes(int n, int64_t batch) {
   if (n < 1 || batch < 0) return 0;
   // reduction matrix and eigenvectors (n^2 each), inverse-iteration scratch
-  // (5 n per eigenvalue, whole warps), d/e, their QL copies and the sorted
-  // eigenvalues, limits (4), FP32 copy of T
+  // (5 n per eigenvalue, whole warps), d/e, their scaled copies and the sorted
+  // eigenvalues, limits (4) and the scale, FP32 copy of T
   return (((size_t)7 * n * n + (size_t)5 * n) * (size_t)batch + (size_t)5 * 32 * n +
-          (size_t)4 * batch + (size_t)n * batch) * sizeof(double);
+          (size_t)5 * batch + (size_t)n * batch) * sizeof(double);
 }
 
 extern "C" int qsx_eigh_large_batched(const double* H, int n, int64_t batch, double* E,
@@ -723,7 +764,8 @@ extern "C" int qsx_eigh_large_batched(const double* H, int n, int64_t batch, dou
   double* tri = de + 2 * (size_t)n * batch;
   double* ws = de + 4 * (size_t)n * batch;
   double* lim = ws + (size_t)n * batch;
-  float* trif = (float*)(lim + 4 * (size_t)batch);
+  double* expo = lim + 4 * (size_t)batch;
+  float* trif = (float*)(expo + batch);
   int dev = 0, sms = 0;
   cudaError_t err = cudaGetDevice(&dev);
   if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -756,14 +798,14 @@ extern "C" int qsx_eigh_large_batched(const double* H, int n, int64_t batch, dou
     err = cudaFuncSetAttribute(eigh_tridiag_cluster_kernel,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemA);
     if (err == cudaSuccess)
-      err = cudaLaunchKernelEx(&cfg, eigh_tridiag_cluster_kernel, H, n, c, W, de);
+      err = cudaLaunchKernelEx(&cfg, eigh_tridiag_cluster_kernel, H, n, c, W, de, expo);
   } else {
     const int threads = n >= TQ_THREADS ? TQ_THREADS : ((n + 31) / 32) * 32;
     const size_t smem = ((size_t)2 * n + 32) * sizeof(double);
     err = cudaFuncSetAttribute(eigh_tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem);
     if (err == cudaSuccess)
-      eigh_tridiag_kernel<<<(unsigned)batch, threads, smem, s>>>(H, n, W, de);
+      eigh_tridiag_kernel<<<(unsigned)batch, threads, smem, s>>>(H, n, W, de, expo);
   }
   if (err != cudaSuccess) return cuda_status(err, "qsx_eigh_large_batched");
   const int64_t nt = batch * n;
@@ -789,7 +831,7 @@ extern "C" int qsx_eigh_large_batched(const double* H, int n, int64_t batch, dou
     const int64_t nn = (int64_t)n * n;
     eigh_backtransform_kernel<<<dim3((unsigned)((n + cols - 1) / cols), (unsigned)nb),
                                 (cols * parts + 31) / 32 * 32, smemD, s>>>(
-        W + b0 * nn, ws + b0 * n, n, cols, parts, Z + b0 * nn, E + b0 * n, U + b0 * nn);
+        W + b0 * nn, ws + b0 * n, expo + b0, n, cols, parts, Z + b0 * nn, E + b0 * n, U + b0 * nn);
   }
   QSX_LAUNCH_CHECK("qsx_eigh_large_batched");
   return QSX_OK;
