@@ -389,19 +389,20 @@ __global__ void __launch_bounds__(128)
   const double* d = de + b * 2 * (int64_t)n;
   const double* e = d + n;
   double lo = d[0], hi = d[0], tnorm = 0.0;
+  bool bad = false;
   for (int i = lane; i < n; i += 32) {
     const double r = (i ? fabs(e[i - 1]) : 0.0) + fabs(e[i]);
     lo = fmin(lo, d[i] - r);
     hi = fmax(hi, d[i] + r);
     tnorm = fmax(tnorm, fabs(d[i]) + r);
-    if (!isfinite(d[i]) || !isfinite(e[i])) tnorm = nan("");   // kept by the test below
+    bad |= !isfinite(d[i]) || !isfinite(e[i]);
   }
   for (int o = 16; o; o >>= 1) {
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    const double t = __shfl_xor_sync(0xffffffffu, tnorm, o);
-    tnorm = isnan(t) || isnan(tnorm) ? nan("") : fmax(tnorm, t);
+    tnorm = fmax(tnorm, __shfl_xor_sync(0xffffffffu, tnorm, o));
   }
+  if (__any_sync(0xffffffffu, bad)) tnorm = nan("");   // (fmax drops a NaN)
   int ex = 0;
   if (tnorm > 0.0 && isfinite(tnorm)) ex = max(-1000, min(1000, ilogb(tnorm)));
   for (int i = lane; i < n; i += 32) {

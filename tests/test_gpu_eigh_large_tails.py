@@ -26,3 +26,13 @@ def test_small_elements_below_a_large_one(n, tail, scale):
     assert np.abs(E - np.linalg.eigvalsh(A)).max() < 4 * n * 2.3e-16 * norm
     assert np.abs(A @ U - U * E).max() < 1e-11 * norm
     assert np.abs(U.T @ U - np.eye(n)).max() < 1e-10
+
+
+@pytest.mark.parametrize('n', [40, 600])
+@pytest.mark.parametrize('where', [(0, 0), (3, 1), (30, 2)])
+@pytest.mark.parametrize('value', [float('nan'), float('inf')])
+def test_a_non_finite_element_is_reported(n, where, value):
+    A = np.eye(n) + np.eye(n, k=1) + np.eye(n, k=-1)
+    A[where] = A[where[::-1]] = value
+    with pytest.raises(_native.QsxError):
+        _native.eigh_large(torch.as_tensor(A)[None].cuda())
