@@ -880,6 +880,19 @@ def _rk4_check(st):
         raise QsxError('qsx_rk4_batched: index table out of range')
 
 
+def rk4_doubles(m, outputs, save_every):
+    """Whether the library takes the states of one m-element FP64 trajectory,
+    ``outputs`` of them after the first, by doubling (it asks for a workspace
+    then) and not step by step."""
+    a = Rk4Args()
+    a.precision, a.m, a.batch = QSX_FP64, m, 1
+    a.nsteps, a.save_every = outputs * save_every, save_every
+    a.matrix = a.y0 = a.out_state = 16     # not read by the query
+    nbytes = ctypes.c_size_t(0)
+    return (load().qsx_rk4_workspace_bytes(ctypes.byref(a), ctypes.byref(nbytes)) == 0
+            and nbytes.value > 0)
+
+
 def rk4(matrix, y0, nsteps, save_every=1, form=0, h=0.0, precision=None,
         state=False, proj=None, select=None, per_sample=True, mean=False,
         check_finite=True, workspace=None, block_k=0, variant=0, later=None):

@@ -147,11 +147,36 @@ def integrate(f, y0, t, t0=None, method_name='rk4', f_params=None,
     return state.cpu().numpy() if as_numpy else state
 
 
-# Hierarchies whose dense propagator pays: a 252-element trimer's square is
-# 0.11 ms and its D 0.1 ms, a stage of the stepped loop 6 us (four a step);
-# past 400 elements the squares cost more than the stages they replace.
+# The dense propagator of small hierarchies: not past this size, nor below this
+# many steps (64 steps are 0.3 to 0.6 ms of the loop, a dense call 0.5 at least)
 HEOM_DENSE_MAX = 400
 HEOM_DENSE_STEPS = 64
+HEOM_DENSE_BLOCK = 1 << 24       # state elements of a block of outputs (256 MB)
+
+
+def _heom_dense_pays(tb, nsteps, every, precision):
+    """Whether the states by doubling of the dense propagator come sooner than
+    the loop over the hierarchy, and the doubling takes them.
+
+    Times of a call in us, fitted to 19 hierarchies of 12 to 576 elements and 16
+    to 4000 steps.  Loop: 180 and, a step, 4 + 3 a coupling term of a node in
+    FP64 (2 sites of one mode 10.4, 7 sites 26.8), in FP32 3 + 1.45 a term through
+    the cluster kernel and 5.3 on chip.  Dense: 500, and 7.5e-6 dim^3 for each
+    product of two propagators: those that make the propagator of ``every``
+    steps, and past 16 outputs a square whenever the outputs double (252
+    elements: 0.53 ms for 16 steps, 1.2 for 256; 392 elements 0.58 and 2.3)."""
+    dim = tb.nnodes * tb.nx * tb.ny
+    outputs = nsteps // every + 1
+    if (dim > HEOM_DENSE_MAX or nsteps < HEOM_DENSE_STEPS
+            or not _native.rk4_doubles(dim, min(outputs, HEOM_DENSE_BLOCK // dim) - 1, every)):
+        return False
+    products = every.bit_length() + bin(every).count('1') - 2 + max(0.0, np.log2(outputs) - 4)
+    step_us = 4 + 3 * tb.nterms
+    if precision == _native.QSX_FP32:
+        on_chip = (3 <= tb.nx == tb.ny <= 8 and 1 <= tb.nterms <= 2 * tb.n_sites
+                   and tb.gamma is None)
+        step_us = 5.3 if on_chip else 3 + 1.45 * tb.nterms
+    return 500 + 7.5e-6 * dim ** 3 * products < 180 + step_us * nsteps
 
 
 def _heom_propagator(f, h):
@@ -165,6 +190,31 @@ def _heom_propagator(f, h):
         z = _native.heom_rhs(f.tables, f.Hx, f.Hy, z if k == 4 else eye + z,
                              f.model.unit_convert) * (h / k)
     return z.T.contiguous()
+
+
+def _heom_dense(f, y, nsteps, every, step, nodes):
+    """(1, outputs, nodes nx ny) states through the dense propagator, in equal
+    blocks of outputs: of the other nodes' states a block is kept at a time."""
+    D = _heom_propagator(f, step)
+    keep = nodes * f.tables.nx * f.tables.ny
+    rest = nsteps // every               # outputs after the first
+    blocks = -(-rest // (HEOM_DENSE_BLOCK // f.dim - 1))
+    out, at = None, 0
+    y = y.contiguous()
+    for k in range(blocks):
+        end = rest * (k + 1) // blocks
+        state = _native.rk4(D, y, (end - at) * every, every, precision=_native.QSX_FP64,
+                            state=True, check_finite=False)['state']
+        if blocks == 1:
+            out = state[..., :keep].contiguous()
+        else:
+            if out is None:
+                out = state.new_empty((1, rest + 1, keep))
+            out[:, at:end + 1] = state[..., :keep]
+            y, at = state[0, -1].clone(), end
+    if not bool(torch.isfinite(torch.view_as_real(out)).all()):
+        raise _native.IntegratorError('non-finite state during HEOM integration')
+    return out
 
 
 def _integrate_heom(f, y0, t, t0, save_func, precision, step, heom_nodes):
@@ -188,20 +238,17 @@ def _integrate_heom(f, y0, t, t0, save_func, precision, step, heom_nodes):
     squeeze = y.dim() == 1
     Y = y[None] if squeeze else y.reshape(-1, y.shape[-1])
     B = Y.shape[0] if f.Hx.dim() == 2 else f.Hx.shape[0]
-    if B == 1 and f.Hx.dim() == 2 and f.dim <= HEOM_DENSE_MAX and nsteps >= HEOM_DENSE_STEPS:
+    prec = _precision(precision)
+    every = max(every, 1)
+    if (B == 1 and f.Hx.dim() == 2 and 1 <= nodes <= tb.nnodes
+            and _heom_dense_pays(tb, nsteps, every, prec)):
         # a small hierarchy: its RK4 propagator as one dense matrix, the
         # states by doubling (every SM) instead of a barrier a stage
-        D = _heom_propagator(f, step)
-        state = _native.rk4(D, Y[0].contiguous(), nsteps, max(every, 1),
-                            precision=_native.QSX_FP64, state=True,
-                            check_finite=False)['state']
-        res = {'state': state[..., :nodes * tb.nx * tb.ny].contiguous()}
-        if not bool(torch.isfinite(torch.view_as_real(res['state'])).all()):
-            raise _native.IntegratorError('non-finite state during HEOM integration')
+        res = {'state': _heom_dense(f, Y[0], nsteps, every, step, nodes)}
     else:
         res = _native.heom_rk4(tb, f.Hx, f.Hy, Y if Y.shape[0] > 1 else Y[0], nsteps, step,
-                               f.model.unit_convert, batch=B, save_every=max(every, 1),
-                               save_nodes=nodes, precision=_precision(precision))
+                               f.model.unit_convert, batch=B, save_every=every,
+                               save_nodes=nodes, precision=prec)
     state = res['state']
     if save_func is not None:
         if not isinstance(save_func, LinearMap):
