@@ -49,7 +49,7 @@ def build(verbose=False, force=False):
     """Compile every .cu under csrc/ and link libqsx.so; returns its path."""
     os.makedirs(OUT_DIR, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC)
-               if f.endswith('.cuh')]
+               if f.endswith(('.cuh', '.h'))]
     headers.append(os.path.join(os.path.dirname(HERE), 'include', 'qsx.h'))
     srcs = sources()
     objs = [os.path.join(OUT_DIR, os.path.basename(s)[:-3] + '.o') for s in srcs]

@@ -31,6 +31,7 @@
 // the wavefronts to conflicts, 28% are left (neighbours at arbitrary places).
 #include <algorithm>
 
+#include "cluster_choice.h"
 #include "heom_site.cuh"
 
 namespace qsx {
@@ -484,9 +485,6 @@ bool hs_launch(HsP p, cudaStream_t s, int* st) {
     const int np = (p.nnodes + c - 1) / c;
     return np <= HS_SLOTS * NPP && hs_smem_bytes<NB>(np, p.n_sites) <= most;
   };
-  int c = 1;
-  while (c < HS_MAX_CLUSTER && !fits(c)) c *= 2;
-  if (!fits(c)) return false;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   cfg.blockDim = dim3(HS_THREADS);
@@ -507,18 +505,16 @@ bool hs_launch(HsP p, cudaStream_t s, int* st) {
                              (int)cfg.dynamicSmemBytes);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveClusters(&clusters, heom_site_kernel<NB>, &cfg);
-    return e == cudaSuccess ? clusters : 0;
-  };
-  int clusters = configure(c);
-  if (e == cudaSuccess && clusters < 1) return false;   // cannot be scheduled here
-  // twice the CTAs a sample while all samples still run at once
-  while (e == cudaSuccess && c < HS_MAX_CLUSTER && p.nnodes > c * NPP) {
-    if (configure(2 * c) < p.batch) {
-      if (e == cudaSuccess) configure(c);
-      break;
+    if (e != cudaSuccess) {
+      cudaGetLastError();   // the other forms of the loop still run
+      e = cudaSuccess;
+      clusters = 0;
     }
-    c *= 2;
-  }
+    return clusters;
+  };
+  const int c = choose_cluster(p.batch, HS_MAX_CLUSTER, fits,
+                               [&](int size) { return p.nnodes > size * NPP; }, configure);
+  if (!c || configure(c) < 1) return false;
   const size_t osmem = (size_t)p.nnodes * 12;
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(hs_order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
