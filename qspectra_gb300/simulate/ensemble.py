@@ -242,8 +242,8 @@ def pick_block_k_real(nsteps, m, nselect, max_k=64, tensor_core=None):
 
 # Measured choice of K for the real blocked loop: the candidates the cost
 # model ranks best are timed once (block build plus loop, on the first call's
-# own inputs) per (m, selected coordinates, steps, batch octave), and the
-# fastest is kept for the process.  set_block_k_real(K) pins a value.
+# own inputs) per (m, selected coordinates, steps, batch octave), and
+# _measured_choice's is kept for the process.  set_block_k_real(K) pins a value.
 _TUNED_K_REAL = {}
 _PINNED_K_REAL = None
 K_REAL_CANDIDATES = 5
@@ -265,6 +265,37 @@ def block_k_real_candidates(nsteps, m, nselect, tensor_core=None, count=K_REAL_C
     return [K for _, K in sorted(ranked)[:count]]
 
 
+# Rounding of the tensor-core build (3xTF32 products that do not round every add
+# to nearest) grows with K and is the same way in every sample, the CUDA-core
+# build's is not.  Against 64 bits, population means of 7 sites at 1000 steps:
+# K = 2 5.8e-8, 5 1.8e-7, 9 3.1e-7, 17 5.7e-7; CUDA cores at K = 2 to 5 1.3e-8.
+# So the tuner's K of that build ends at 9, although 16 is sooner (16384
+# samples, build and loop: 0.96 ms and 1.10), and a CUDA-core candidate goes
+# before a tensor-core one that is less than a tenth sooner (5 sites, every
+# component, 2001 samples: K = 6 0.283 ms and 2.0e-8, K = 5 0.262 and 5.2e-8).
+TC_BUILD_MAX_K = 9
+TC_BUILD_GAIN = 0.9
+
+
+def _tensor_core_build(m, K, nselect):
+    """Whether the blocked matrix of K steps is built on the tensor cores (a
+    pinned K wherever the shape allows)."""
+    return ((K <= TC_BUILD_MAX_K or K == _PINNED_K_REAL)
+            and _native.rk4_block_matrix_real_tc_supported(m, K, nselect))
+
+
+def _measured_choice(times, tensor_core):
+    """K from {K: ms}; ``tensor_core(K)`` as in pick_block_k_real, or None."""
+    tc = [K for K in times if tensor_core is not None and tensor_core(K)]
+    fast = min(times, key=times.get)
+    rest = [K for K in times if K not in tc]
+    if fast in tc and rest:
+        other = min(rest, key=times.get)
+        if times[fast] > TC_BUILD_GAIN * times[other]:
+            return other
+    return fast
+
+
 def _real_block_pass(Dr, K, coords, x0, nsteps, use_tc):
     tc = _native.rk4_block_matrix_real_tc(Dr, K, coords) if use_tc else None
     if tc is not None:
@@ -280,8 +311,7 @@ def tuned_block_k_real(Dr, coords, x0, nsteps, use_tc):
     """K for the real blocked loop: pinned, measured once per shape, or (while
     a CUDA graph is being captured, where nothing can be timed) the model's."""
     m = int(Dr.shape[-1])
-    tcf = ((lambda k: _native.rk4_block_matrix_real_tc_supported(m, k, len(coords)))
-           if use_tc else None)
+    tcf = (lambda k: _tensor_core_build(m, k, len(coords))) if use_tc else None
     if _PINNED_K_REAL is not None:
         return _PINNED_K_REAL
     key = (m, len(coords), int(nsteps), int(np.log2(max(int(Dr.shape[0]), 1))), bool(use_tc))
@@ -302,7 +332,7 @@ def tuned_block_k_real(Dr, coords, x0, nsteps, use_tc):
         e1.record()
         e1.synchronize()
         times[K] = e0.elapsed_time(e1)
-    best = min(times, key=times.get)
+    best = _measured_choice(times, tcf)
     _TUNED_K_REAL[key] = (best, times)
     return best
 
@@ -366,7 +396,7 @@ def propagate_hermitian_mean(build, idx, nb, h, y0, nsteps, select, events=None,
     if x0 is None:
         x0 = hermitian_coordinates(y0, nb)
     K = tuned_block_k_real(Dr, coords, x0, nsteps, use_tc)
-    use_tc = use_tc and bool(_native.rk4_block_matrix_real_tc_supported(m, K, len(coords)))
+    use_tc = use_tc and _tensor_core_build(m, K, len(coords))
     if events is not None:
         b0 = torch.cuda.Event(enable_timing=True)
         b0.record()
