@@ -140,13 +140,15 @@ __global__ void __launch_bounds__(256)
 // t3; any strides) over t1 and t3 in one launch (FP64):
 //   X[k1][b][k3] = dt1 dt3 sum_{n1, n3} x[n1][b][n3]
 //                  exp(i s1 (f1_k1 - rw) uc t1_n1) exp(i s3 (f3_k3 - rw) uc t3_n3),
-//                  exp(i s1 (f1_k1 - rw) uc t1_n1) exp(i s3 (f3_k3 - rw) uc t3_n3),
 // t_n = t0 + n dt on each axis.  CTA (chunk of F3 t3 frequencies, b): first the
 // t3 transform of every t1 row for those frequencies, into shared memory
 // (Y[n1][F3]); then the t1 transform of Y for every t1 frequency.  The bound is
-// each SM's FP64 pipe, so F3 is the largest of 8, 4, 2 with a CTA for every SM: a
-// 100 x 3 x 100 signal on 199 x 199 frequencies took 652 us in 75 CTAs with
-// rotated twiddles, 173 in 150.
+// each SM's FP64 pipe: a CTA costs as F3 (n1 = n3 = 100: 85, 160 and 310 us for
+// 2, 4 and 8), and those on one SM share it, so F3 is the one of 8, 4, 2 whose
+// busiest SM has the least to do (the largest of equals, which repeats the fewest
+// loads).  us with F3 = 8, 4, 2 on 152 SMs: 64 x 5 x 64 140, 143, 118; 100 x 3 x
+// 100 321, 175, 173 (652 with rotated twiddles); 100 x 4 x 100 320, 315, 252; 128 x
+// 5 x 128 908, 691, 593; 60 x 3 x 200 195, 205, 224.
 template <int F3>
 __global__ void __launch_bounds__(256)
     dft2_kernel(const double2* __restrict__ x, int n1, int n3, int64_t s1, int64_t sb,
@@ -247,8 +249,11 @@ extern "C" int qsx_dft2_batched(const double* x, int n1, int64_t batch, int n3, 
     QSX_LAUNCH_CHECK("qsx_dft2_batched");
     return QSX_OK;
   };
-  auto ctas = [&](int chunk) { return (int64_t)((nf3 + chunk - 1) / chunk) * batch; };
-  if (ctas(8) >= sms) return run(qsx::dft2_kernel<8>, 8);
-  // 150 CTAs for 152 SMs are enough
-  return ctas(4) >= sms - sms / 8 ? run(qsx::dft2_kernel<4>, 4) : run(qsx::dft2_kernel<2>, 2);
+  // the busiest SM's frequencies
+  auto load = [&](int chunk) {
+    return ((int64_t)((nf3 + chunk - 1) / chunk) * batch + sms - 1) / sms * chunk;
+  };
+  const int64_t l8 = load(8), l4 = load(4), l2 = load(2);
+  if (l8 <= l4 && l8 <= l2) return run(qsx::dft2_kernel<8>, 8);
+  return l4 <= l2 ? run(qsx::dft2_kernel<4>, 4) : run(qsx::dft2_kernel<2>, 2);
 }
