@@ -210,7 +210,7 @@ def _rk4_step_arrays(L, h):
 def rk4_step_minus_identity(L, h):
     """D = P - I, P = sum_{k<=4} (hL)^k / k! (Paterson-Stockmeyer form)."""
     if (L.is_cuda and L.dtype == torch.complex128 and L.dim() == 3
-            and L.shape[-2] == L.shape[-1] <= _native.FIT_MAX and isinstance(h, (int, float))
+            and 0 < L.shape[-2] == L.shape[-1] <= _native.FIT_MAX and isinstance(h, (int, float))
             and _native.plain(L)):
         # a copy: the caller may reuse L's memory before the backward pass, and
         # a conjugate view becomes the values themselves

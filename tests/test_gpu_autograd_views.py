@@ -105,3 +105,11 @@ def test_transforms_of_the_step():
     assert err(torch.func.jvp(f, (L,), (t,))[1], want) < 1e-14
     with fwd.dual_level():
         assert err(fwd.unpack_dual(f(fwd.make_dual(L, t))).tangent, want) < 1e-14
+
+
+@pytest.mark.parametrize('shape', [(0, 7, 7), (3, 0, 0), (3, 1, 1)])
+def test_empty_batches_and_blocks_of_the_step(shape):
+    L = draw(*shape).requires_grad_(True)
+    D = adj.rk4_step_minus_identity(L, 0.7)
+    assert D.shape == shape
+    assert torch.autograd.grad(D.real.sum(), L)[0].shape == shape
