@@ -62,13 +62,19 @@ def test_objects_made_on_a_busy_stream_serve_another():
     off = m.hamiltonian.disorder_offsets(64)
     dense = np.random.RandomState(1).randn(40, 30) + 0j
     x = torch.ones(3, 30, dtype=torch.complex128, device='cuda')
-    torch.cuda.synchronize()
     a, b = torch.cuda.Stream(), torch.cuda.Stream()
-    with torch.cuda.stream(a):
-        torch.cuda._sleep(100_000_000)      # about 50 ms
-        batch, table = SampleBatch(m, 64), _native.CsrMap(dense)
-    with torch.cuda.stream(b):
-        H, y = batch.H('e'), table(x)
-        H, y = H.cpu().numpy(), y.cpu().numpy()
+    for busy in (False, True):      # once to have the memory, which waits for the GPU
+        with torch.cuda.stream(a):
+            if busy:
+                torch.cuda._sleep(400_000_000)      # about 0.2 s
+            batch, table = SampleBatch(m, 64), _native.CsrMap(dense)
+        with torch.cuda.stream(b):
+            H, y = batch.H('e'), table(x)
+            H, y = H.cpu().numpy(), y.cpu().numpy()
+        if not busy:
+            batch.offsets.zero_()
+            table.vals.zero_()
+            del batch, table
+            torch.cuda.synchronize()
     np.testing.assert_allclose(H, expected(m, off, 'e'), rtol=1e-13)
     np.testing.assert_allclose(y, np.repeat(dense.sum(1)[None], 3, 0), rtol=1e-13)
