@@ -1331,7 +1331,8 @@ def _eigh_check(st):
 
 
 def eigh_large(H, later=None):
-    """Batched FP64 eigensolver (Householder + implicit QL) for any n <= 2048.
+    """Batched FP64 eigensolver (Householder, bisection and inverse iteration)
+    for any n <= 2048.
     H (B, n, n) float64 CUDA, symmetric.  Returns E ascending and U."""
     require_gpu()
     _need(H, torch.float64, 'H', 3)

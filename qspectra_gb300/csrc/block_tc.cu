@@ -24,7 +24,7 @@
 // a CTA took 118 KB at K = 17, so that one ran on an SM; now two do from 70 KB
 // each.  Bound: the latency of a phase, about 1700 cycles of MMAs and 2000 of
 // the D warps' epilogue, two CTAs under each other.  16384 samples of m = 49,
-// seven rows: K = 9 740 us before, K = 17 1300 before and 498 here.
+// seven rows: K = 9 740 us before and 490 here, K = 17 1300 and 498.
 //
 // The kernel is persistent: each CTA loops over samples, keeps its tensor
 // memory, barrier and zero padding, and prefetches the next sample's D with

@@ -11,8 +11,9 @@
 // this one, 495 nodes of 8 x 8: 36.4 / 16.0 for 64 samples, 21.8 / 8.2 for 32,
 // 7.3 / 5.2 for one.  Against the cluster form of heom.cu (what ran small
 // hierarchies): 3.1 / 2.9 for one sample of 120 nodes of 3 x 3, 15.0 / 2.9 for
-// 64; 9.2 / 3.0 and 17.7 (per-stage) / 4.3 with 120 nodes of 7 x 7.  Every
-// size measured from 4 to 495 nodes and 1 to 300 samples is faster here.
+// 64; 9.2 / 3.0 and 17.7 (per-stage) / 4.3 with 120 nodes of 7 x 7.  Every one
+// of 68 sizes measured, 3 to 8 sites, 4 to 495 nodes and 1 to 300 samples, is
+// faster here.
 //
 // A thread owns a 2 x 2 tile of a node's block, the same tile for up to four
 // nodes, with its two rows of Hx and two columns of Hy in registers.  With

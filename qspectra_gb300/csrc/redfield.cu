@@ -156,6 +156,12 @@ __global__ void __launch_bounds__(64)
 //   the tangents to FP32 accuracy (an element shrinks by 1e-7 a rotation, the
 //   quadratic convergence does the same), cosines in FP64.
 // The matrix is scaled by a power of two into FP32's range.
+// Accuracy: E to a few ulp of the largest element, U orthonormal to FP64 rounding
+// (half the residual of the thread form on 4200 random matrices).  X^T A X is
+// formed in FP64, so an eigenvalue far below the norm has the norm's absolute
+// error: the relative one that FP64 Jacobi sweeps keep on graded matrices (levels
+// of very different sizes with couplings to match) is not kept.  Energies enter
+// the generators by their differences alone.
 template <int NB>
 struct EighWarpSmem {
   static constexpr int LD = NB + 1;
@@ -166,7 +172,8 @@ constexpr int EIGH_BLOCK_WARPS = 2;
 // is about NB^3 long and hidden by the other matrices once they fill the chip,
 // where a warp per matrix spends more FP64 issue slots.  Measured, thread form
 // and warp form: 3 x 3, 10000 matrices 65 / 241 us; 7 x 7, 300: 403 / 57,
-// 10000: 498 / 560, 200000: 4588 / 9499; 8 x 8, 10000: 743 / 662.
+// 10000: 498 / 560, 200000: 4588 / 9499; 8 x 8, 10000: 743 / 662.  (So the last
+// bits of a sample's eigenpairs depend on the size of its batch.)
 template <int NB>
 constexpr int64_t EIGH_WARP_MAX = 19 * NB * NB * NB;
 
@@ -443,7 +450,7 @@ __global__ void __launch_bounds__(32 * EIGH_BLOCK_WARPS)
 // equal p + q together: they share no state, and of two pairs that do the one
 // with the smaller sum comes first by rows as well, so that the result is that
 // of the row order (signs and places of the eigenvectors, blocks that stay
-// apart).  A warp a matrix, one rotation after the other in FP64, took 4.0 ms
+// apart).  Accuracy as there: E to ulp of the norm.  A warp a matrix, one rotation after the other in FP64, took 4.0 ms
 // for 32 matrices of 25 states, 0.45 here (9 states 0.45 and 0.12; 10000 matrices
 // of 25 states 67 and 9.2 ms).
 constexpr int EIGH_MID_THREADS = 256, EIGH_LD = EIGH_NMAX + 1;

@@ -14,7 +14,7 @@
 //
 // simulate_dynamics of 300 7-site samples, 499 steps: 5.66 ms with the complex
 // loop (a CTA per sample, two barriers a step) and its propagators, 2.36 ms
-// with the real ones.
+// with the real ones (1.89 ms as the call is now, the loop 1.04 of it).
 #include <algorithm>
 
 #include "qsx_common.cuh"

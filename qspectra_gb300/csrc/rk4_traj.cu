@@ -17,11 +17,14 @@
 // with coalesced loads of DT and broadcast loads of x.
 //
 // Bound: FP64 issue (2 multiply-adds per clock and SM) once a phase fills the
-// chip, launch latency before that.  Whole calls in FP64, before and after: a
-// 7-site trajectory (49 elements, 1000 states) 8.52 and 0.45 ms, a 7-site
-// spectrum (7 elements, 2048 states) 5.11 and 1.24 ms, a dimer trajectory (4
-// elements, 120 states) 0.51 and 0.35 ms, a trimer hierarchy through its
-// dense propagator (252 elements, 500 states) 12.6 and 1.65 ms.
+// chip, launch latency before that.  Whole calls in FP64, with the stepped loop
+// and as they are now: a 7-site trajectory (49 elements, 1000 states) 8.52 and
+// 0.42 ms, a 7-site spectrum (7 elements, 2048 states) 5.11 and 0.82 ms, a dimer
+// trajectory (4 elements, 120 states) 0.51 and 0.32 ms, a trimer hierarchy
+// through its dense propagator (252 elements, 500 states) 12.6 and 1.64 ms.
+// Rounding: a few ulp more than the steps leave (error against 64-bit formulas
+// 9e-16 and 1.5e-15 for the 7 sites, 2e-16 and 7e-16 for the trimer), as the
+// powers' own rounding is shared by the states of a block.
 //
 // A power can overflow, or meet a non-finite generator, where the stepped
 // loop would not (an unstable mode that the state does not excite).  Every

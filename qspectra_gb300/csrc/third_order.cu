@@ -377,7 +377,10 @@ __global__ void __launch_bounds__(FE_THREADS, 1) fe_loop_kernel(FeP p, FeLoop l)
 constexpr int FE_TEAM_WARPS = 8, FE_TEAM_THREADS = 32 * FE_TEAM_WARPS;
 constexpr int FE_TEAM_CT = 8;     // columns of a row-term task
 constexpr int FE_TEAM_RREG = 6;   // FP32 rows that a warp can keep in registers
-constexpr int FE_TEAM_NQ[3] = {4, 6, 9};   // terms a lane, of up to 128, 192, 288 pairs
+// Terms a lane, of up to 128, 192 and 288 pairs (24 sites).  Past nine the six
+// register rows and a lane's part of X no longer fit: 236 registers at nine, 255
+// and spills at ten.  25 to 31 sites take the loop over the L2.
+constexpr int FE_TEAM_NQ[3] = {4, 6, 9};
 
 struct FeTeam {
   int64_t batch, y0_stride;

@@ -9,8 +9,8 @@ block-diagonal over the g/e/f manifolds, so this engine never forms the
 
 * g and e blocks come from a 'ge' Redfield build (batched FP64 Jacobi
   eigensolve and operator-form tensor, one CTA per sample);
-* the f manifold is diagonalised per sample (FP64 Householder + QL kernel),
-  its eigenbasis tensor
+* the f manifold is diagonalised per sample (``qsx_eigh_large_batched``:
+  FP64 Householder, bisection, inverse iteration), its eigenbasis tensor
   Kt_i o C is built in FP64 by ``qsx_fblock_tensor``, and two batched GEMMs
   bring M_i^f to the site basis in the working precision;
 * t1 and the 'eg' t3 leg run in the batched RK4 kernels; the t2 leg applies
