@@ -598,9 +598,9 @@ int qsx_zofe_rk4(const qsx_zofe_args* args, void* stream);
 /*
  * Batched FP64 symmetric eigensolver for n up to 2048 (the two-exciton
  * block; the reference calls scipy.linalg.eigh per sample,
- * qspectra/hamiltonian.py:310-328): Householder tridiagonalisation (one CTA
- * per matrix), bisection on Sturm counts and inverse iteration (one thread
- * per eigenvalue), back-transform by the reflectors.  H float64 [batch][n][n] symmetric;
+ * qspectra/hamiltonian.py:310-328): Householder tridiagonalisation (a cluster
+ * of CTAs per matrix), bisection on Sturm counts and inverse iteration (one
+ * thread per eigenvalue), back-transform by the reflectors.  H float64 [batch][n][n] symmetric;
  * E float64 [batch][n] ascending; U float64 [batch][n][n], column k the
  * eigenvector of E[k].  Workspace: qsx_eigh_large_workspace_bytes.
  * status: QSX_ERR_NONFINITE when an eigenvalue comes out non-finite.
